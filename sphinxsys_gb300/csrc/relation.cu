@@ -9,8 +9,8 @@
 //
 // Storage is ELL, slot-major: entry s of source particle i sits at s * n_src + i, so a
 // warp of consecutive particles reads slot s of all its lanes in one coalesced access.
-// Per entry: neighbour index j, dW_ij, e_ij (dim components), and r_ij / W_ij when the
-// relation needs them.  Inner relations also keep sigma_i = W0 + sum_j W_ij and contact
+// Per entry: neighbour index j, dW_ij, e_ij (dim components; in fixed point for inner
+// relations, fx.cuh), and r_ij / W_ij when the relation needs them.  Inner relations also keep sigma_i = W0 + sum_j W_ij and contact
 // relations sum_j W_ij m_j / rho0_j, the two sums DensitySummation needs
 // (density_summation.cpp:74-82,113-122).
 //
@@ -19,7 +19,9 @@
 // oracle's bit for bit.  An FP32 test on cell-relative offsets first rejects candidates
 // clearly outside the cut-off.
 #include <algorithm>
+#include <cstring>
 
+#include "fx.cuh"
 #include "sphx_device.cuh"
 #include "sphx_internal.cuh"
 
@@ -42,10 +44,12 @@ struct BuildArgs
     int depth, cap;
     uint32_t *count, *J;
     double *DW, *E, *R, *W; // E: dim arrays of cap * n_src
+    fx::EntryStore fx;      // inner relations: in place of DW and E
     double *wsum;
     const double *tgt_mass;
     double tgt_inv_rho0;
-    unsigned int *max_count;
+    unsigned int *max_count; // [0] longest list, [1] source particles with neighbours (contact)
+    uint32_t *active;
 };
 
 // Two passes per source particle.  Pass 1 walks the candidate cells with the FP32
@@ -142,13 +146,25 @@ __global__ void __launch_bounds__(kBlock) k_build(BuildArgs a)
         double t = 1.0 - 0.5 * q;
         double t2 = t * t, t3 = t2 * t;
         double W = a.k.factor_W * (t2 * t2 * (1.0 + 2.0 * q));
-        double dW = a.k.factor_dW * (-5.0 * t3 * q);
+        double K = -5.0 * t3 * q;
         size_t slot = size_t(cnt) * a.n_src + i;
         a.J[slot] = j;
-        a.DW[slot] = dW;
+        if (INNER)
+        {
+            fx::Entry<D> q;
+            q.k = fx::encode(K);
 #pragma unroll
-        for (int d = 0; d < D; ++d)
-            a.E[d * stride + slot] = dx[d] * inv;
+            for (int d = 0; d < D; ++d)
+                q.e[d] = fx::encode(dx[d] * inv);
+            a.fx.store<D>(slot, q);
+        }
+        else
+        {
+            a.DW[slot] = a.k.factor_dW * K;
+#pragma unroll
+            for (int d = 0; d < D; ++d)
+                a.E[d * stride + slot] = dx[d] * inv;
+        }
         if (a.R)
             a.R[slot] = r;
         if (a.W)
@@ -162,6 +178,8 @@ __global__ void __launch_bounds__(kBlock) k_build(BuildArgs a)
     a.count[i] = cnt;
     a.wsum[i] = ws;
     warp_atomic_max(a.max_count, cand);
+    if (!INNER && cnt > 0)
+        a.active[atomicAdd(a.max_count + 1, 1u)] = uint32_t(i);
 }
 } // namespace
 
@@ -174,8 +192,19 @@ void sphx_relation_s::release()
     cudaFree(r);
     cudaFree(e);
     cudaFree(wsum);
-    count = j = nullptr;
-    dW = W = r = e = wsum = nullptr;
+    cudaFree(fx_rec);
+    cudaFree(fx_k);
+    cudaFree(active);
+    cudaFree(contact_sum);
+    cudaFree(fx_value);
+    cudaFree(fx_flag);
+    count = j = fx_flag = active = nullptr;
+    dW = W = r = e = wsum = contact_sum = nullptr;
+    fx_rec = nullptr;
+    fx_k = nullptr;
+    n_active = 0;
+    fx_value = nullptr;
+    fx_epoch[0] = fx_epoch[1] = 0;
     cap = 0;
     n_src = 0;
 }
@@ -190,8 +219,22 @@ int sphx_relation_s::allocate(int new_cap, size_t n)
     SPHX_CUDA(cudaMalloc(&count, nn * sizeof(uint32_t)));
     SPHX_CUDA(cudaMalloc(&wsum, nn * sizeof(double)));
     SPHX_CUDA(cudaMalloc(&j, slots * sizeof(uint32_t)));
-    SPHX_CUDA(cudaMalloc(&dW, slots * sizeof(double)));
-    SPHX_CUDA(cudaMalloc(&e, slots * dim * sizeof(double)));
+    if (inner)
+    {
+        SPHX_CUDA(cudaMalloc(&fx_rec, slots * (dim == 2 ? 1 : 2) * sizeof(int4)));
+        if (dim == 2)
+            SPHX_CUDA(cudaMalloc(&fx_k, slots * sizeof(int2)));
+        SPHX_CUDA(cudaMalloc(&fx_value, nn * (dim == 2 ? 2 : 4) * sizeof(long long)));
+        SPHX_CUDA(cudaMalloc(&fx_flag, 2 * sizeof(uint32_t)));
+        SPHX_CUDA(cudaMemsetAsync(fx_flag, 0, 2 * sizeof(uint32_t), ctx->stream));
+    }
+    else
+    {
+        SPHX_CUDA(cudaMalloc(&dW, slots * sizeof(double)));
+        SPHX_CUDA(cudaMalloc(&e, slots * dim * sizeof(double)));
+        SPHX_CUDA(cudaMalloc(&active, nn * sizeof(uint32_t)));
+        SPHX_CUDA(cudaMalloc(&contact_sum, nn * (dim + 1) * sizeof(double)));
+    }
     if (store_r)
         SPHX_CUDA(cudaMalloc(&r, slots * sizeof(double)));
     if (store_W)
@@ -293,6 +336,8 @@ static int launch_build(sphx_relation rel, unsigned int *d_max)
     a.J = rel->j;
     a.DW = rel->dW;
     a.E = rel->e;
+    a.fx = fx::EntryStore{rel->fx_rec, rel->fx_k};
+    a.active = rel->active;
     a.R = rel->r;
     a.W = rel->W;
     a.wsum = rel->wsum;
@@ -334,11 +379,13 @@ extern "C" int sphx_relation_update(sphx_relation rel)
     unsigned int *d_max = reinterpret_cast<unsigned int *>(ctx->d_red);
     for (int attempt = 0; attempt < 2; ++attempt)
     {
-        SPHX_CUDA(cudaMemsetAsync(d_max, 0, sizeof(unsigned int), ctx->stream));
+        SPHX_CUDA(cudaMemsetAsync(d_max, 0, 2 * sizeof(unsigned int), ctx->stream));
         SPHX_TRY(launch_build(rel, d_max));
-        SPHX_CUDA(cudaMemcpyAsync(ctx->h_red, d_max, sizeof(unsigned int), cudaMemcpyDeviceToHost, ctx->stream));
+        SPHX_CUDA(cudaMemcpyAsync(ctx->h_red, d_max, 2 * sizeof(unsigned int), cudaMemcpyDeviceToHost, ctx->stream));
         SPHX_CUDA(cudaStreamSynchronize(ctx->stream));
-        unsigned int maxc = *reinterpret_cast<unsigned int *>(ctx->h_red);
+        const unsigned int *built = reinterpret_cast<unsigned int *>(ctx->h_red);
+        const unsigned int maxc = built[0];
+        rel->n_active = built[1];
         if (maxc <= unsigned(rel->cap))
             return SPHX_OK;
         // grow with head room and search again
@@ -360,12 +407,19 @@ extern "C" int sphx_relation_download(sphx_relation rel, uint32_t *counts, uint3
         SPHX_CUDA(cudaMemcpyAsync(cnt.data(), rel->count, n * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
     size_t slots = size_t(rel->cap) * n;
     std::vector<uint32_t> hj(j ? slots : 0);
-    std::vector<double> hW(W && rel->W ? slots : 0), hdW(dW ? slots : 0), hr(r && rel->r ? slots : 0),
-        he(e ? slots * dim : 0);
+    std::vector<double> hW(W && rel->W ? slots : 0), hdW(dW && !rel->inner ? slots : 0),
+        hr(r && rel->r ? slots : 0), he(e && !rel->inner ? slots * dim : 0);
     if (j && slots)
         SPHX_CUDA(cudaMemcpyAsync(hj.data(), rel->j, slots * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
     if (!hW.empty())
         SPHX_CUDA(cudaMemcpyAsync(hW.data(), rel->W, slots * sizeof(double), cudaMemcpyDeviceToHost, s));
+    // an inner relation's entries are fixed-point words: K and e together in 3D
+    std::vector<int4> hrec(rel->inner && (dW || e) ? slots * (dim == 2 ? 1 : 2) : 0);
+    std::vector<int2> hk(rel->inner && dim == 2 && dW ? slots : 0);
+    if (!hrec.empty())
+        SPHX_CUDA(cudaMemcpyAsync(hrec.data(), rel->fx_rec, hrec.size() * sizeof(int4), cudaMemcpyDeviceToHost, s));
+    if (!hk.empty())
+        SPHX_CUDA(cudaMemcpyAsync(hk.data(), rel->fx_k, hk.size() * sizeof(int2), cudaMemcpyDeviceToHost, s));
     if (!hdW.empty())
         SPHX_CUDA(cudaMemcpyAsync(hdW.data(), rel->dW, slots * sizeof(double), cudaMemcpyDeviceToHost, s));
     if (!hr.empty())
@@ -373,6 +427,14 @@ extern "C" int sphx_relation_download(sphx_relation rel, uint32_t *counts, uint3
     if (!he.empty())
         SPHX_CUDA(cudaMemcpyAsync(he.data(), rel->e, slots * dim * sizeof(double), cudaMemcpyDeviceToHost, s));
     SPHX_CUDA(cudaStreamSynchronize(s));
+    const double factor_dW = wendland(dim, rel->h).factor_dW;
+    // word w of an entry: 0 the kernel derivative, 1 + d the unit vector's component d
+    auto word = [&](size_t slot, int w) {
+        if (dim == 2 && w == 0)
+            return fx::decode(hk[slot]);
+        const int2 *q = reinterpret_cast<const int2 *>(hrec.data());
+        return fx::decode(dim == 2 ? q[2 * slot + (w - 1)] : q[4 * slot + w]);
+    };
     size_t t = 0;
     for (size_t i = 0; i < n; ++i)
     {
@@ -385,13 +447,15 @@ extern "C" int sphx_relation_download(sphx_relation rel, uint32_t *counts, uint3
                 j[t] = hj[slot];
             if (!hW.empty())
                 W[t] = hW[slot];
-            if (!hdW.empty())
+            if (dW && rel->inner)
+                dW[t] = factor_dW * word(slot, 0);
+            else if (!hdW.empty())
                 dW[t] = hdW[slot];
             if (!hr.empty())
                 r[t] = hr[slot];
-            if (!he.empty())
+            if (e)
                 for (int d = 0; d < dim; ++d)
-                    e[t * dim + d] = he[d * slots + slot];
+                    e[t * dim + d] = rel->inner ? word(slot, 1 + d) : he[d * slots + slot];
         }
     }
     if (total)

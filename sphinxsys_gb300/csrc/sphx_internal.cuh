@@ -159,6 +159,19 @@ struct sphx_relation_s
     uint32_t *j = nullptr;
     double *dW = nullptr, *W = nullptr, *r = nullptr, *e = nullptr;
     double *wsum = nullptr; // inner: W0 + sum W; contact: sum W inv_rho0 m_j
+    // Inner relations hold the kernel derivative (over its prefactor) and the unit vector in
+    // fixed point instead of dW and e (fx.cuh), and a workspace for the particle values of a
+    // sweep with the verdict of its conversion.
+    int4 *fx_rec = nullptr;
+    int2 *fx_k = nullptr; // 2D
+    long long *fx_value = nullptr;
+    uint32_t *fx_flag = nullptr; // one word per half step
+    uint32_t fx_epoch[2] = {0, 0};
+    // Contact relations: the source particles with neighbours (n_active of them, in no
+    // order) and a workspace for their sums.
+    uint32_t *active = nullptr;
+    size_t n_active = 0;
+    double *contact_sum = nullptr; // (dim + 1) x n_src
     int allocate(int cap, size_t n_src);
     void release();
 };
