@@ -443,7 +443,7 @@ __device__ __forceinline__ void fixed_2nd(size_t n, size_t i, unsigned sub, cons
             const bool capped = T > lim;
             const int bh = capped ? int(lim >> 31) : max(th, 0);
             const int bl = capped ? int(unsigned(lim) & 0x7fffffffu) : (th < 0 ? 0 : tl);
-            const long long sm = fx::mad(av, bh, fx::mad(ah, bl, 0));
+            const long long sm = fx::mad(av, bh, fx::mad(ah, bl, 1 << 24));
             const long long sc = (fx::mad(ah, bh, 0) << 6) + (sm >> 25); // in units of 2^56
             const int sh = int(sc >> 31), sl = int(unsigned(sc) & 0x7fffffffu);
 #pragma unroll

@@ -202,6 +202,94 @@ struct EntryStore
     }
 };
 
+// ---------------------------------------------------------------- pair geometry
+// Halves of a non-negative value below 2^62 for products: v = h 2^31 + l.
+struct Halves
+{
+    int h, l;
+};
+__device__ __forceinline__ Halves halves(long long v) { return {int(v >> 31), int(unsigned(v) & 0x7fffffffu)}; }
+// a b / 2^31 - (a.h b.h) 2^31, the two upper parts of a product (a may be negative)
+__device__ __forceinline__ long long middle(Halves a, Halves b, long long round = 0)
+{
+    return mad(a.h, b.l, mad(a.l, b.h, round)) + (mad(a.l, b.l, 0) >> 31);
+}
+// a b / 2^57 for 0 <= a, b <= 2^57
+__device__ __forceinline__ long long product57(Halves a, Halves b)
+{
+    return (mad(a.h, b.h, 0) << 5) + (middle(a, b, 1 << 25) >> 26);
+}
+__device__ __forceinline__ int2 split(long long v) // halves of a list entry
+{
+    const int l = int(unsigned(v) << 1) >> 1;
+    return make_int2(int((v - l) >> 31), l);
+}
+
+// Constants of the pair geometry of one kernel: positions in units of 2^unit, differences
+// shifted left by `shift` so that the cut-off lies in [2^58, 2^59); inv_rc = 2^118 / cut-off.
+struct GeometryScale
+{
+    int unit, shift;
+    long long inv_rc;
+};
+
+// Wendland C2 of one pair in fixed point: D = x_i - x_j in the shifted units.  Writes the
+// entry (kernel derivative over its prefactor, unit vector), r over the cut-off in units of
+// 2^-57 and the kernel over its prefactor in units of 2^-54.  Returns false (nothing written)
+// for points closer than about 1/16 of the cut-off, which take the FP64 form.
+//
+// 1 / |D| comes from the hardware's FP32 reciprocal root of the leading bits and one
+// third-order Newton step, y = y0 (1 + e / 2 + 3 e^2 / 8) with the residual
+// e = 1 - |D|^2 y0^2 formed exactly to 2^-64; |e| < 2^-20 leaves e^3 below 2^-60.
+template <int D>
+__device__ __forceinline__ bool wendland_pair(const long long *dx, const GeometryScale &g, Entry<D> &out,
+                                              long long &r57, long long &w54)
+{
+    long long hh = 0, m = 0, ll = 0;
+#pragma unroll
+    for (int d = 0; d < D; ++d)
+    {
+        const int h = int(dx[d] >> 30), l = int(unsigned(dx[d]) & 0x3fffffffu);
+        hh = mad(h, h, hh);
+        m = mad(h, l, m);
+        ll = mad(l, l, ll);
+    }
+    // |D|^2 / 2^58
+    const long long z = (hh << 2) + ((m + (ll >> 31)) >> 27);
+    if (z < (1ll << 51))
+        return false;
+    const int half = (__clzll(z) - 2) >> 1;
+    const long long R = z << (2 * half); // [2^60, 2^62)
+    const float y0 = rsqrtf(float(int(R >> 32)));
+    const int Y0 = __float2int_rn(y0 * 274877906944.0f); // 2^38: 1 / sqrt(R / 2^62) in units of 2^-23
+    const Halves Rh = halves(R), q = halves(mad(Y0, Y0, 0));
+    // 2^64 (1 - R Y0^2 / 2^108), modulo 2^64
+    const long long E = -((mad(Rh.h, q.h, 0) << 18) + (middle(Rh, q) >> 13));
+    const int es = int(E >> 20);
+    const long long C = (E >> 1) + ((mad(es, es, 0) * 3) >> 27);
+    // units of 2^-58
+    const long long Y = (static_cast<long long>(Y0) << 35) +
+                        (mad(Y0, int(C >> 16), mad(Y0, int(C & 0xffff), 0) >> 16) >> 13);
+    const Halves Yh = halves(Y);
+    // sqrt(R / 2^62) in units of 2^-58, then r / cut-off in units of 2^-57
+    const long long root = mad(Rh.h, Yh.h, 0) + (middle(Rh, Yh, 1 << 30) >> 31);
+    const Halves rt = halves(root), ic = halves(g.inv_rc);
+    r57 = ((mad(rt.h, ic.h, 0) << 3) + (middle(rt, ic, 1 << 27) >> 28)) >> half;
+#pragma unroll
+    for (int d = 0; d < D; ++d)
+    {
+        const Halves n = halves(dx[d] << half);
+        out.e[d] = split((mad(n.h, Yh.h, 0) << 1) + (middle(n, Yh, 1 << 29) >> 30));
+    }
+    // t = 1 - r / rc, q = 2 r / rc: dW ~ -5 t^3 q, W ~ t^4 (1 + 2 q)
+    const Halves t = halves(max((1ll << 57) - r57, 0ll)), rr = halves(r57);
+    const Halves t2 = halves(product57(t, t)), t3 = halves(product57(t2, t));
+    out.k = split(-10 * product57(t3, rr));
+    const long long t4 = product57(t2, t2);
+    w54 = (t4 + 4 * product57(halves(t4), rr) + 4) >> 3;
+    return true;
+}
+
 // Sums over the LANES threads of a particle.
 template <int LANES>
 __device__ __forceinline__ unsigned group_mask()

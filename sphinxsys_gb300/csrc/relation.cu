@@ -16,10 +16,16 @@
 //
 // Membership test: |x_i - x_j|^2 < (2h)^2 in FP64 with the canonical association
 // ((dx*dx + dy*dy) + dz*dz) and no fused multiply-add, so the pair set equals the
-// oracle's bit for bit.  An FP32 test on cell-relative offsets first rejects candidates
-// clearly outside the cut-off.
+// oracle's bit for bit.  An FP32 test on cell-relative offsets decides all candidates but
+// those within its own rounding of the cut-off, which take the FP64 test.
+//
+// The update is two kernels: the search writes each particle's candidate entries, the second
+// one the values of the accepted pairs: in fixed point for inner relations (fx.cuh), in FP64
+// by 8 threads per particle with neighbours for contact relations.
 #include <algorithm>
+#include <cmath>
 #include <cstring>
+#include <limits>
 
 #include "fx.cuh"
 #include "sphx_device.cuh"
@@ -42,9 +48,14 @@ struct BuildArgs
     MeshDev m;
     WendlandC2 k;
     int depth, cap;
+    float accept_sqr, reject_sqr, self_sqr; // bounds of the FP32 test (see search_bounds)
     uint32_t *count, *J;
     double *DW, *E, *R, *W; // E: dim arrays of cap * n_src
     fx::EntryStore fx;      // inner relations: in place of DW and E
+    const longlong4_32a *fx_pos; // inner relations: {x, y, z, particle} of the cell-list entries
+    fx::GeometryScale g;
+    uint32_t *fx_flag;
+    uint32_t fx_epoch;
     double *wsum;
     const double *tgt_mass;
     double tgt_inv_rho0;
@@ -52,134 +63,338 @@ struct BuildArgs
     uint32_t *active;
 };
 
-// Two passes per source particle.  Pass 1 walks the candidate cells with the FP32
-// pre-filter only and writes the cell-list entry index of every candidate that passes
-// into the particle's list slots.  Pass 2 walks that short list: the exact FP64 membership
-// test, then W, dW, e (and r) in FP64 for the accepted pairs, compacted in place.  The FP64
-// work of pass 2 runs with nearly all lanes of a warp busy; in one pass it ran for the
-// whole warp whenever any lane accepted a candidate.  Entries, order and values are those
-// of the one-pass form.  The capacity check uses the pass-1 count (a superset).
-template <int D, bool INNER>
-__global__ void __launch_bounds__(kBlock) k_build(BuildArgs a)
+__device__ __forceinline__ void load_position(const double *x, size_t n, size_t i, int dim, double *out)
 {
-    size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i >= a.n_src)
-        return;
-    double xi[3] = {0, 0, 0};
+    for (int d = 0; d < dim; ++d)
+        out[d] = x[d * n + i];
+}
+
+// The exact membership test; its square distance in r2.
+template <int D>
+__device__ __forceinline__ bool within(const BuildArgs &a, const double *xi, uint32_t kk, double *dx, double &r2)
+{
 #pragma unroll
     for (int d = 0; d < D; ++d)
-        xi[d] = a.src_pos[d * a.n_src + i];
+        dx[d] = __dsub_rn(xi[d], a.spos[d * a.n_tgt + kk]);
+    r2 = __dadd_rn(__dmul_rn(dx[0], dx[0]), __dmul_rn(dx[1], dx[1]));
+    if (D == 3)
+        r2 = __dadd_rn(r2, __dmul_rn(dx[2], dx[2]));
+    return r2 < a.k.rc_sqr;
+}
+
+// The test for the search, out of line: inlined, the compiler predicates its FP64
+// instructions instead of branching around them, and every candidate pays for them (wall
+// search of 1,702,400 particles 16 ms).
+template <int D>
+__device__ __noinline__ bool exact_test(const double *x_i, const double *spos, size_t n_tgt, uint32_t kk, size_t n_src,
+                                        double rc_sqr)
+{
+    double r2 = 0.0;
+    for (int d = 0; d < D; ++d)
+    {
+        const double dx = __dsub_rn(x_i[d * n_src], spos[d * n_tgt + kk]);
+        r2 = d == 0 ? __dmul_rn(dx, dx) : __dadd_rn(r2, __dmul_rn(dx, dx));
+    }
+    return r2 < rc_sqr;
+}
+
+// The search: LANES threads per particle test the candidates of a cell side by side and
+// append the accepted ones in cell order (a ballot gives each its slot).  One thread per
+// particle keeps the list writes of a warp together and does the least work per candidate;
+// few particles need the threads to cover the memory latency.
+template <int D, bool INNER, int LANES>
+__global__ void __launch_bounds__(kBlock) k_build(BuildArgs a)
+{
+    const size_t g = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
+    const bool live = g / LANES < a.n_src;
+    const size_t i = live ? g / LANES : a.n_src - 1; // threads past the end repeat the last particle
+    const unsigned sub = unsigned(g % LANES);
+    double xi[3] = {0, 0, 0};
+    load_position(a.src_pos, a.n_src, i, D, xi);
     int c[3] = {0, 0, 0}, lo[3] = {0, 0, 0}, hi[3] = {1, 1, 1};
     cell_index<D>(a.m, xi, c);
+    // offset from the corner of the first cell of the window along each axis
+    float o[3] = {0, 0, 0};
+    const float gs = float(a.m.gs);
+    bool inside = true;
 #pragma unroll
     for (int d = 0; d < D; ++d)
     {
         lo[d] = max(0, c[d] - a.depth);
         hi[d] = min(a.m.all_cells[d], c[d] + a.depth + 1);
+        o[d] = float(xi[d] - cell_corner(a.m, d, lo[d]));
+        const float own = o[d] - float(c[d] - lo[d]) * gs;
+        inside = inside && own > -0.5f * gs && own < 1.5f * gs;
     }
-    const size_t stride = size_t(a.cap) * a.n_src;
-    // pass 1: FP32 pre-filter, candidate entries into the list slots
-    unsigned cand = 0;
+    // a particle outside the mesh sits far from its cell's corner: every candidate below the
+    // wide bound takes the exact test
+    const float accept = inside ? a.accept_sqr : -1.0f;
+    const float reject = inside ? a.reject_sqr : a.k.prefilter_sqr;
+    const unsigned lane = threadIdx.x & 31u;
+    const unsigned group = LANES == 1 ? 0u : fx::group_mask<LANES>();
+    unsigned cnt = 0;
     int cc[3] = {0, 0, 0};
     for (cc[0] = lo[0]; cc[0] < hi[0]; ++cc[0])
     {
-        float o0 = float(xi[0] - cell_corner(a.m, 0, cc[0]));
-        for (cc[1] = lo[1]; cc[1] < hi[1]; ++cc[1])
+        const float o0 = fmaf(-float(cc[0] - lo[0]), gs, o[0]);
+        // 2D: the column of cells along axis 1; 3D: a column along axis 2 for every cc[1]
+        for (cc[1] = lo[1]; cc[1] < (D == 3 ? hi[1] : lo[1] + 1); ++cc[1])
         {
-            float o1 = float(xi[1] - cell_corner(a.m, 1, cc[1]));
-            for (cc[2] = lo[2]; cc[2] < hi[2]; ++cc[2])
+            const float o1 = D == 3 ? fmaf(-float(cc[1] - lo[1]), gs, o[1]) : 0.0f;
+            cc[2] = lo[2];
+            const int cells = hi[D - 1] - lo[D - 1];
+            const uint32_t first = linear_cell<D>(a.m, cc);
+            uint32_t ke = a.cell_offset[first];
+            if (a.cell_offset[first + cells] == ke)
+                continue;
+            for (int k = 0; k < cells; ++k)
             {
-                float o2 = D == 3 ? float(xi[2] - cell_corner(a.m, 2, cc[2])) : 0.0f;
-                uint32_t lc = linear_cell<D>(a.m, cc);
-                uint32_t kb = a.cell_offset[lc], ke = a.cell_offset[lc + 1];
+                const float ol = fmaf(-float(k), gs, o[D - 1]);
+                uint32_t kb = ke;
+                ke = a.cell_offset[first + k + 1];
+                uint32_t stop = ke;
                 if (!SPHX_CHECKED(kb <= ke && ke <= a.n_tgt, kCheckCellRange, (uint64_t(kb) << 32) | ke))
-                    ke = kb;
-                for (uint32_t kk = kb; kk < ke; ++kk)
+                    stop = kb;
+                for (uint32_t kk = kb + sub; LANES == 1 ? kk < stop : kk - sub < stop; kk += LANES)
                 {
-                    float f0 = o0 - a.soff[kk], f1 = o1 - a.soff[a.n_tgt + kk];
-                    float d2f = f0 * f0 + f1 * f1;
-                    if (D == 3)
+                    bool take = LANES == 1 || kk < stop;
+                    if (take)
                     {
-                        float f2 = o2 - a.soff[2 * a.n_tgt + kk];
-                        d2f += f2 * f2;
+                        const float f0 = o0 - a.soff[kk];
+                        const float f1 = (D == 3 ? o1 : ol) - a.soff[a.n_tgt + kk];
+                        float d2 = f0 * f0 + f1 * f1;
+                        if (D == 3)
+                        {
+                            const float f2 = ol - a.soff[2 * a.n_tgt + kk];
+                            d2 += f2 * f2;
+                        }
+                        take = d2 < reject;
+                        if (take && !(d2 < accept))
+                            take = exact_test<D>(a.src_pos + i, a.spos, a.n_tgt, kk, a.n_src, a.k.rc_sqr);
+                        if (INNER && take && (!inside || d2 < a.self_sqr))
+                            take = a.pidx[kk] != uint32_t(i);
                     }
-                    if (d2f > a.k.prefilter_sqr)
-                        continue;
-                    if (INNER && a.pidx[kk] == uint32_t(i))
-                        continue;
-                    if (cand < unsigned(a.cap))
-                        a.J[size_t(cand) * a.n_src + i] = kk;
-                    ++cand;
+                    unsigned slot = cnt;
+                    if (LANES == 1)
+                        cnt += take ? 1u : 0u;
+                    else
+                    {
+                        const unsigned votes = __ballot_sync(group, take) & group;
+                        slot += __popc(votes & ((1u << lane) - 1u));
+                        cnt += __popc(votes);
+                    }
+                    if (take && live && slot < unsigned(a.cap))
+                        a.J[size_t(slot) * a.n_src + i] = kk;
                 }
-                if (D == 2)
-                    break;
             }
         }
     }
-    // pass 2: exact test and kernel values over the candidates, in place
-    const unsigned stored = min(cand, unsigned(a.cap));
-    unsigned cnt = 0;
-    double ws = INNER ? a.k.factor_W : 0.0;
-    for (unsigned s = 0; s < stored; ++s)
+    const bool writes = live && sub == 0;
+    if (writes)
+        a.count[i] = min(cnt, unsigned(a.cap));
+    warp_atomic_max(a.max_count, live ? cnt : 0u);
+    if (INNER)
+        return;
+    // the particles with neighbours, one global atomic per block (one per particle made the
+    // search of 1,702,400 particles take 16 ms)
+    __shared__ unsigned found, base;
+    if (threadIdx.x == 0)
+        found = 0;
+    __syncthreads();
+    unsigned place = 0;
+    if (writes)
     {
-        const uint32_t kk = a.J[size_t(s) * a.n_src + i];
+        a.wsum[i] = 0.0;
+        if (cnt > 0)
+            place = atomicAdd(&found, 1u);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0 && found > 0)
+        base = atomicAdd(a.max_count + 1, found);
+    __syncthreads();
+    if (writes && cnt > 0)
+        a.active[base + place] = uint32_t(i);
+}
+
+// One pair in FP64: the square distance gives W, dW, e and r.
+template <int D>
+__device__ __forceinline__ void pair_fp64(const BuildArgs &a, double r2, double &W, double &K, double &r, double &inv)
+{
+    // one reciprocal square root gives r and 1/r; e = dx / (r + TinyReal) of the
+    // reference differs from dx / r by TinyReal / r relative, far below one rounding,
+    // except for coincident particles where e is zero
+    const double ri = rsqrt(r2);
+    r = r2 > 0.0 ? r2 * ri : 0.0;
+    inv = r2 > 0.0 ? ri : 1.0 / kTinyReal;
+    const double q = r * a.k.inv_h;
+    // Wendland C2 with t = 1 - q/2: W ~ t^4 (1 + 2q), dW ~ 0.625 (q - 2)^3 q = -5 t^3 q
+    const double t = 1.0 - 0.5 * q;
+    const double t2 = t * t;
+    W = t2 * t2 * (1.0 + 2.0 * q);
+    K = -5.0 * (t2 * t) * q;
+}
+template <int D>
+__device__ __noinline__ void entry_fp64(const BuildArgs &a, size_t i, uint32_t kk, fx::Entry<D> &q, long long &r57,
+                                        long long &w54)
+{
+    double xi[3], dx[3], r2, W, K, r, inv;
+    load_position(a.src_pos, a.n_src, i, D, xi);
+    within<D>(a, xi, kk, dx, r2);
+    pair_fp64<D>(a, r2, W, K, r, inv);
+    q.k = fx::encode(K);
+    for (int d = 0; d < D; ++d)
+        q.e[d] = fx::encode(dx[d] * inv);
+    r57 = __double2ll_rn(r * (0.5 * a.k.inv_h) * fx::pow2(57));
+    w54 = __double2ll_rn(W * fx::pow2(54));
+}
+
+// The cell-list entries' positions in units of 2^unit with their particle: what a pair reads
+// of its neighbour, in one record.
+template <int D>
+__global__ void k_fix_positions(size_t n, const double *__restrict__ spos, const uint32_t *__restrict__ pidx, int unit,
+                                longlong4_32a *__restrict__ out, uint32_t *flag, uint32_t epoch)
+{
+    const size_t k = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
+    if (k >= n)
+        return;
+    bool fits = true;
+    long long q[3] = {0, 0, 0};
+#pragma unroll
+    for (int d = 0; d < D; ++d)
+        q[d] = fx::fixed(spos[d * n + k], unit, fits);
+    longlong2 *rec = reinterpret_cast<longlong2 *>(out + k);
+    rec[0] = make_longlong2(q[0], q[1]);
+    rec[1] = make_longlong2(q[2], static_cast<long long>(pidx[k]));
+    if (!fits)
+        *flag = epoch;
+}
+
+// Values of the pairs of an inner relation.  In FP64 a pair costs about 45 instructions of
+// the FP64 pipe (720 cycles of an SM per warp); in fixed point about 50 wide multiply-adds
+// and 150 other integer instructions.  Search and values of 1,702,400 particles (130 M
+// pairs): 8.3 ms in FP64, 1.9 + 2.3 ms here.
+template <int D, int LANES>
+__global__ void __launch_bounds__(kBlock) k_pairs_inner(BuildArgs a)
+{
+    const size_t g = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
+    const size_t i = g / LANES;
+    const unsigned sub = unsigned(g % LANES);
+    if (i >= a.n_src)
+        return;
+    bool fixed = __ldcg(a.fx_flag) != a.fx_epoch;
+    long long x_i[3] = {0, 0, 0};
+#pragma unroll
+    for (int d = 0; d < D; ++d)
+        x_i[d] = fx::fixed(a.src_pos[d * a.n_src + i], a.g.unit, fixed);
+    const unsigned cnt = a.count[i];
+    long long w_sum = 0; // at most 256 terms of up to 2^54
+    double w_total = 0.0;
+    for (unsigned s = sub, term = 0; s < cnt; s += LANES, ++term)
+    {
+        if ((term & 0xff) == 0xff)
+        {
+            w_total += double(w_sum);
+            w_sum = 0;
+        }
+        const size_t slot = size_t(s) * a.n_src + i;
+        const uint32_t kk = a.J[slot];
         if (!SPHX_CHECKED(kk < a.n_tgt && a.pidx[kk] < a.n_tgt, kCheckListEntry, kk))
             continue;
-        double dx[3] = {0, 0, 0};
-#pragma unroll
-        for (int d = 0; d < D; ++d)
-            dx[d] = __dsub_rn(xi[d], a.spos[d * a.n_tgt + kk]);
-        double r2 = __dadd_rn(__dmul_rn(dx[0], dx[0]), __dmul_rn(dx[1], dx[1]));
-        if (D == 3)
-            r2 = __dadd_rn(r2, __dmul_rn(dx[2], dx[2]));
-        if (!(r2 < a.k.rc_sqr))
-            continue;
-        const uint32_t j = a.pidx[kk];
-        // one reciprocal square root gives r and 1/r; e = dx / (r + TinyReal) of the
-        // reference differs from dx / r by TinyReal / r relative, far below one rounding,
-        // except for coincident particles where e is zero
-        double ri = rsqrt(r2);
-        double r = r2 > 0.0 ? r2 * ri : 0.0;
-        double inv = r2 > 0.0 ? ri : 1.0 / kTinyReal;
-        double q = r * a.k.inv_h;
-        // Wendland C2 with t = 1 - q/2: W ~ t^4 (1 + 2q), dW ~ 0.625 (q - 2)^3 q = -5 t^3 q
-        double t = 1.0 - 0.5 * q;
-        double t2 = t * t, t3 = t2 * t;
-        double W = a.k.factor_W * (t2 * t2 * (1.0 + 2.0 * q));
-        double K = -5.0 * t3 * q;
-        size_t slot = size_t(cnt) * a.n_src + i;
-        a.J[slot] = j;
-        if (INNER)
+        const longlong2 *rec = reinterpret_cast<const longlong2 *>(a.fx_pos + kk);
+        const longlong2 p = __ldg(rec), w = __ldg(rec + 1);
+        const long long dx[3] = {(x_i[0] - p.x) << a.g.shift, (x_i[1] - p.y) << a.g.shift,
+                                 (x_i[2] - w.x) << a.g.shift};
+        fx::Entry<D> q;
+        long long r57, w54;
+        if (!fixed || !fx::wendland_pair<D>(dx, a.g, q, r57, w54))
+            entry_fp64<D>(a, i, kk, q, r57, w54);
+        a.J[slot] = uint32_t(w.y);
+        a.fx.store<D>(slot, q);
+        if (a.R)
+            a.R[slot] = double(r57) * (2.0 * a.k.h * fx::pow2(-57));
+        w_sum += w54;
+    }
+    w_total = fx::group_sum<LANES>(w_total + double(w_sum));
+    if (sub == 0)
+        a.wsum[i] = a.k.factor_W * (1.0 + w_total * fx::pow2(-54));
+}
+
+// Values of the pairs of a contact relation: kContactLanes threads per particle that has any.
+constexpr int kContactLanes = 8;
+template <int D>
+__global__ void __launch_bounds__(kBlock) k_pairs_contact(BuildArgs a)
+{
+    const size_t stride = size_t(a.cap) * a.n_src;
+    const unsigned n_active = __ldcg(a.max_count + 1);
+    const size_t groups = size_t(gridDim.x) * blockDim.x / kContactLanes;
+    const size_t g = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
+    const unsigned sub = unsigned(g % kContactLanes);
+    for (size_t k = g / kContactLanes; k < n_active; k += groups)
+    {
+        const size_t i = a.active[k];
+        double xi[3] = {0, 0, 0};
+        load_position(a.src_pos, a.n_src, i, D, xi);
+        const unsigned cnt = a.count[i];
+        double ws = 0.0;
+        for (unsigned s = sub; s < cnt; s += kContactLanes)
         {
-            fx::Entry<D> q;
-            q.k = fx::encode(K);
-#pragma unroll
-            for (int d = 0; d < D; ++d)
-                q.e[d] = fx::encode(dx[d] * inv);
-            a.fx.store<D>(slot, q);
-        }
-        else
-        {
+            const size_t slot = size_t(s) * a.n_src + i;
+            const uint32_t kk = a.J[slot];
+            if (!SPHX_CHECKED(kk < a.n_tgt && a.pidx[kk] < a.n_tgt, kCheckListEntry, kk))
+                continue;
+            double dx[3], r2, W, K, r, inv;
+            within<D>(a, xi, kk, dx, r2);
+            pair_fp64<D>(a, r2, W, K, r, inv);
+            const uint32_t j = a.pidx[kk];
+            W *= a.k.factor_W;
+            a.J[slot] = j;
             a.DW[slot] = a.k.factor_dW * K;
 #pragma unroll
             for (int d = 0; d < D; ++d)
                 a.E[d * stride + slot] = dx[d] * inv;
-        }
-        if (a.R)
             a.R[slot] = r;
-        if (a.W)
             a.W[slot] = W;
-        if (INNER)
-            ws += W;
-        else
             ws += (W * a.tgt_inv_rho0) * a.tgt_mass[j];
-        ++cnt;
+        }
+        ws = fx::group_sum<kContactLanes>(ws);
+        if (sub == 0)
+            a.wsum[i] = ws;
     }
-    a.count[i] = cnt;
-    a.wsum[i] = ws;
-    warp_atomic_max(a.max_count, cand);
-    if (!INNER && cnt > 0)
-        a.active[atomicAdd(a.max_count + 1, 1u)] = uint32_t(i);
+}
+
+// Bounds of the FP32 test.  Offsets reach (2 depth + 1) cells of spacing gs and carry up to
+// five roundings, so a squared distance near the cut-off is off by less than
+// 9 (2 depth + 1) (gs / rc) 2^-24 of it; the margin is four times that or more.
+// The particle itself is told from its coincident neighbours by its index, which only near
+// candidates are looked up for; where a periodic image of it can lie within the cut-off, all.
+void search_bounds(BuildArgs &a, const sphx_cell_list_s &cl)
+{
+    const double rc = a.k.rc, m = 64.0 * (a.depth + 1) * std::max(a.m.gs / rc, 1.0) * 0x1p-24;
+    a.accept_sqr = float(a.k.rc_sqr * (1.0 - m));
+    a.reject_sqr = float(a.k.rc_sqr * (1.0 + m));
+    a.self_sqr = float(a.k.rc_sqr * m);
+    for (int d = 0; d < 3; ++d)
+        if ((cl.periodic_mask & (1 << d)) && cl.per_upper[d] - cl.per_lower[d] < 2.0 * rc)
+            a.self_sqr = std::numeric_limits<float>::max();
+}
+
+// Positions up to twice the mesh's corners in 60 bits; differences of up to the cut-off
+// shifted to [2^58, 2^59).  False where the cut-off is too small for the domain (less than
+// 2^-20 of it) to keep its precision.
+bool geometry_scale(const sphx_mesh_desc &m, double rc, fx::GeometryScale &g)
+{
+    double far = 0.0;
+    for (int d = 0; d < m.dim; ++d)
+        far = std::max({far, std::fabs(m.lower[d]), std::fabs(m.lower[d] + m.all_cells[d] * m.grid_spacing)});
+    if (!(far > 0.0) || !std::isfinite(far) || !(rc > 0.0) || !std::isfinite(rc))
+        return false;
+    g.unit = std::ilogb(far) + 2 - 60;
+    g.shift = 58 - (std::ilogb(rc) - g.unit);
+    if (g.shift < 0 || g.shift > 20 || g.unit < -1000 || g.unit > 900)
+        return false;
+    const double cut = std::ldexp(rc, g.shift - g.unit); // [2^58, 2^59)
+    g.inv_rc = std::llrint(std::ldexp(1.0 / std::ldexp(cut, -60), 58));
+    return true;
 }
 } // namespace
 
@@ -198,13 +413,16 @@ void sphx_relation_s::release()
     cudaFree(contact_sum);
     cudaFree(fx_value);
     cudaFree(fx_flag);
+    cudaFree(fx_pos);
+    fx_pos = nullptr;
+    fx_pos_cap = 0;
     count = j = fx_flag = active = nullptr;
     dW = W = r = e = wsum = contact_sum = nullptr;
     fx_rec = nullptr;
     fx_k = nullptr;
     n_active = 0;
     fx_value = nullptr;
-    fx_epoch[0] = fx_epoch[1] = 0;
+    fx_epoch[0] = fx_epoch[1] = fx_epoch[2] = 0;
     cap = 0;
     n_src = 0;
 }
@@ -225,8 +443,8 @@ int sphx_relation_s::allocate(int new_cap, size_t n)
         if (dim == 2)
             SPHX_CUDA(cudaMalloc(&fx_k, slots * sizeof(int2)));
         SPHX_CUDA(cudaMalloc(&fx_value, nn * (dim == 2 ? 2 : 4) * sizeof(long long)));
-        SPHX_CUDA(cudaMalloc(&fx_flag, 2 * sizeof(uint32_t)));
-        SPHX_CUDA(cudaMemsetAsync(fx_flag, 0, 2 * sizeof(uint32_t), ctx->stream));
+        SPHX_CUDA(cudaMalloc(&fx_flag, 3 * sizeof(uint32_t)));
+        SPHX_CUDA(cudaMemsetAsync(fx_flag, 0, 3 * sizeof(uint32_t), ctx->stream));
     }
     else
     {
@@ -332,6 +550,7 @@ static int launch_build(sphx_relation rel, unsigned int *d_max)
     a.k = wendland(src->dim, rel->h);
     a.depth = rel->depth;
     a.cap = rel->cap;
+    search_bounds(a, *cl);
     a.count = rel->count;
     a.J = rel->j;
     a.DW = rel->dW;
@@ -344,22 +563,64 @@ static int launch_build(sphx_relation rel, unsigned int *d_max)
     a.tgt_mass = tmass ? static_cast<const double *>(tmass->dev) : nullptr;
     a.tgt_inv_rho0 = rel->tgt_inv_rho0;
     a.max_count = d_max;
-    unsigned grid = grid_for(a.n_src, kBlock);
-    if (src->dim == 2)
+    const int dim = src->dim;
+    cudaStream_t s = ctx->stream;
+    // threads per particle: 8 until one each gives an SM 512 threads
+    const int lanes = a.n_src < size_t(std::max(1, ctx->num_sms)) * 512 ? 8 : 1;
+    const unsigned grid = grid_for(a.n_src * lanes, kBlock);
+    if (!rel->inner)
     {
-        if (rel->inner)
-            k_build<2, true><<<grid, kBlock, 0, ctx->stream>>>(a);
+        if (dim == 2)
+            lanes == 1 ? k_build<2, false, 1><<<grid, kBlock, 0, s>>>(a) : k_build<2, false, 8><<<grid, kBlock, 0, s>>>(a);
         else
-            k_build<2, false><<<grid, kBlock, 0, ctx->stream>>>(a);
+            lanes == 1 ? k_build<3, false, 1><<<grid, kBlock, 0, s>>>(a) : k_build<3, false, 8><<<grid, kBlock, 0, s>>>(a);
+        SPHX_LAUNCHED(ctx);
+        const unsigned gc = std::min(grid_for(a.n_src * kContactLanes, kBlock), unsigned(std::max(1, ctx->num_sms)) * 8u);
+        if (dim == 2)
+            k_pairs_contact<2><<<gc, kBlock, 0, s>>>(a);
+        else
+            k_pairs_contact<3><<<gc, kBlock, 0, s>>>(a);
+        SPHX_LAUNCHED(ctx);
+        return SPHX_OK;
     }
+    if (dim == 2)
+        lanes == 1 ? k_build<2, true, 1><<<grid, kBlock, 0, s>>>(a) : k_build<2, true, 8><<<grid, kBlock, 0, s>>>(a);
     else
-    {
-        if (rel->inner)
-            k_build<3, true><<<grid, kBlock, 0, ctx->stream>>>(a);
-        else
-            k_build<3, false><<<grid, kBlock, 0, ctx->stream>>>(a);
-    }
+        lanes == 1 ? k_build<3, true, 1><<<grid, kBlock, 0, s>>>(a) : k_build<3, true, 8><<<grid, kBlock, 0, s>>>(a);
     SPHX_LAUNCHED(ctx);
+    SPHX_TRY(rel->reserve_positions(a.n_tgt));
+    a.fx_pos = rel->fx_pos;
+    a.fx_flag = rel->fx_flag + 2;
+    a.fx_epoch = ++rel->fx_epoch[2];
+    // without a scale nothing fits and every pair is taken in FP64
+    const int unit = geometry_scale(cl->mesh, a.k.rc, a.g) ? a.g.unit : -5000;
+    if (dim == 2)
+        k_fix_positions<2><<<grid_for(a.n_tgt, 256), 256, 0, s>>>(a.n_tgt, a.spos, a.pidx, unit, rel->fx_pos,
+                                                                  a.fx_flag, a.fx_epoch);
+    else
+        k_fix_positions<3><<<grid_for(a.n_tgt, 256), 256, 0, s>>>(a.n_tgt, a.spos, a.pidx, unit, rel->fx_pos,
+                                                                  a.fx_flag, a.fx_epoch);
+    SPHX_LAUNCHED(ctx);
+    if (dim == 2)
+        lanes == 1 ? k_pairs_inner<2, 1><<<grid, kBlock, 0, s>>>(a) : k_pairs_inner<2, 8><<<grid, kBlock, 0, s>>>(a);
+    else
+        lanes == 1 ? k_pairs_inner<3, 1><<<grid, kBlock, 0, s>>>(a) : k_pairs_inner<3, 8><<<grid, kBlock, 0, s>>>(a);
+    SPHX_LAUNCHED(ctx);
+    return SPHX_OK;
+}
+
+// The workspace of positions in fixed point, grown with head room.
+int sphx_relation_s::reserve_positions(size_t n)
+{
+    if (n <= fx_pos_cap)
+        return SPHX_OK;
+    cudaStreamSynchronize(ctx->stream);
+    cudaFree(fx_pos);
+    fx_pos = nullptr;
+    fx_pos_cap = 0;
+    const size_t cap_n = n + n / 8;
+    SPHX_CUDA(cudaMalloc(&fx_pos, cap_n * sizeof(longlong4_32a)));
+    fx_pos_cap = cap_n;
     return SPHX_OK;
 }
 

@@ -165,8 +165,11 @@ struct sphx_relation_s
     int4 *fx_rec = nullptr;
     int2 *fx_k = nullptr; // 2D
     long long *fx_value = nullptr;
-    uint32_t *fx_flag = nullptr; // one word per half step
-    uint32_t fx_epoch[2] = {0, 0};
+    uint32_t *fx_flag = nullptr; // one word per half step and one for the pair values
+    uint32_t fx_epoch[3] = {0, 0, 0};
+    longlong4_32a *fx_pos = nullptr; // cell-list entries: position in fixed point, particle
+    size_t fx_pos_cap = 0;
+    int reserve_positions(size_t n);
     // Contact relations: the source particles with neighbours (n_active of them, in no
     // order) and a workspace for their sums.
     uint32_t *active = nullptr;
