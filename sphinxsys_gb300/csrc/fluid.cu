@@ -112,7 +112,15 @@ struct Fixed
     long long *value; // pressure: 1 word a particle; velocity: 2 (2D) or 4 (3D) words
     uint32_t *flag;
     uint32_t epoch;
+    unsigned long long *speed; // epoch and the largest binary exponent of a velocity component
 };
+
+// The unit 2^k of the velocities: their largest component takes 60 bits.
+__device__ __forceinline__ int velocity_unit(const Fixed &f)
+{
+    const int e = int(__ldcg(f.speed) & 0x7ffull);
+    return max(e, 600) - 1022 - fx::kVelocityBits;
+}
 
 struct FluidVars
 {
@@ -164,21 +172,40 @@ __global__ void k_init_1st(size_t n, double *__restrict__ rho, const double *__r
         *fp.flag = fp.epoch;
 }
 
-// Velocities over 2^c0_exp in fixed point, one record of 16 (2D) or 32 (3D) bytes a particle;
-// converted by integer instructions on the bits (the FP64 form of this pass took 47 us for
-// 1,702,400 particles, three times its memory traffic).
 template <int D>
-__global__ void k_init_2nd(size_t n, const double *__restrict__ vel, const double *__restrict__ Vol, int c0_exp,
-                           Fixed fv)
+__global__ void k_largest_velocity(size_t n, const double *__restrict__ vel, Fixed fv)
+{
+    int m = 0;
+    for (size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n * D; i += size_t(gridDim.x) * blockDim.x)
+        m = max(m, __double2hiint(vel[i]) & 0x7fffffff);
+    m = __reduce_max_sync(0xffffffffu, m);
+    __shared__ int sm[32];
+    if ((threadIdx.x & 31u) == 0)
+        sm[threadIdx.x >> 5] = m;
+    __syncthreads();
+    if (threadIdx.x != 0)
+        return;
+    for (unsigned k = 1; k < (blockDim.x >> 5); ++k)
+        m = max(m, sm[k]);
+    // the epoch in front makes the value of every earlier call smaller
+    atomicMax(fv.speed, static_cast<unsigned long long>(fv.epoch) << 11 | unsigned(m >> 20));
+}
+
+// Velocities in fixed point, one record of 16 (2D) or 32 (3D) bytes a particle; converted by
+// integer instructions on the bits (the FP64 form of this pass took 47 us for 1,702,400
+// particles, three times its memory traffic).
+template <int D>
+__global__ void k_init_2nd(size_t n, const double *__restrict__ vel, const double *__restrict__ Vol, Fixed fv)
 {
     size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
     if (i >= n)
         return;
-    bool fits = __double_as_longlong(Vol[i]) == __double_as_longlong(Vol[0]);
+    const int unit = velocity_unit(fv);
+    bool fits = __double_as_longlong(Vol[i]) == __double_as_longlong(Vol[0]) && unit < 400;
     long long q[4] = {0, 0, 0, 0};
 #pragma unroll
     for (int d = 0; d < D; ++d)
-        q[d] = fx::fixed(vel[d * n + i], c0_exp - fx::kVelocityBits, fits);
+        q[d] = fx::fixed(vel[d * n + i], unit, fits);
     longlong2 *out = reinterpret_cast<longlong2 *>(fv.value) + i * (D - 1);
     out[0] = make_longlong2(q[0], q[1]);
     if (D == 3)
@@ -306,10 +333,9 @@ __device__ __forceinline__ void fixed_1st(size_t n, size_t i, unsigned sub, cons
             const int2 K = q[u].k;
             const long long df = P_i - P_j[u], sm = P_i + P_j[u];
             R.add(fx::high(df), fx::low(df), K);
-            R.m = fx::mad(__mulhi(fx::low(df), K.y), 2, R.m);
             const int sh = fx::high(sm), sl = fx::low(sm);
             hh[u] = fx::mad(sh, K.x, 0);
-            m[u] = fx::mad(__mulhi(sl, K.y), 2, 0);
+            m[u] = fx::low_product(sl, K.y, 0);
             m[u] = fx::mad(sh, K.y, m[u]);
             m[u] = fx::mad(sl, K.x, m[u]);
             fx::Align::see(top, hh[u]);
@@ -365,11 +391,11 @@ __device__ __forceinline__ long long limit_at(long long t, int a)
 }
 
 // Integration2ndHalf in fixed point, u = (v_i - v_j) . e: R = sum u K and
-// F = sum u min(u+, u_lim) K e, the dissipation without its constant factors; t_lim is the
-// speed at which the limiter reaches 1, in units of 2^-(55) of the velocity scale.
+// F = sum u min(u+, u_lim) K e, the dissipation without its constant factors; u_lim is the
+// speed at which the limiter reaches 1.
 template <int D, int LANES>
 __device__ __forceinline__ void fixed_2nd(size_t n, size_t i, unsigned sub, const InnerPairs &in,
-                                          const long long *__restrict__ V, long long t_lim, double *force,
+                                          const long long *__restrict__ V, int unit, double u_lim, double *force,
                                           double *rate)
 {
     constexpr int U = LANES == 1 ? kUnroll2 : 2;
@@ -383,6 +409,9 @@ __device__ __forceinline__ void fixed_2nd(size_t n, size_t i, unsigned sub, cons
     }
     fx::Sum F[D], R;
     fx::Align al;
+    // u at alignment 0 is in units of 2^(63 - kListBits + unit)
+    const double l = u_lim * fx::pow2(fx::kListBits - 63 - unit);
+    const long long t_lim = l < 1.0e17 ? __double2ll_rn(l) : 1ll << 57;
     long long lim = 0;
     int folded = 0;
     bool first = true;
@@ -435,16 +464,18 @@ __device__ __forceinline__ void fixed_2nd(size_t n, size_t i, unsigned sub, cons
             const int2 K = q[u].k;
             const long long T = al.apply(hh[u], m[u]); // u
             const int th = int(T >> 31), tl = int(unsigned(T) & 0x7fffffffu);
-            const long long wh = fx::mad(th, K.x, 0), wm = fx::mad(tl, K.x, fx::mad(th, K.y, 0));
-            R.hh += wh;
-            R.m += wm;
-            const long long w = (wh << 5) + (wm >> 26); // u K in units of 2^57
-            const int ah = int(w >> 31), av = int(unsigned(w) & 0x7fffffffu);
+            // u K in units of 2^57
+            const long long wm = fx::low_product(tl, K.y, fx::mad(tl, K.x, fx::mad(th, K.y, 1 << 25)));
+            const long long w = (fx::mad(th, K.x, 0) << 5) + (wm >> 26);
+            R.m += w;
+            // min(u+, limit)
             const bool capped = T > lim;
             const int bh = capped ? int(lim >> 31) : max(th, 0);
             const int bl = capped ? int(unsigned(lim) & 0x7fffffffu) : (th < 0 ? 0 : tl);
-            const long long sm = fx::mad(av, bh, fx::mad(ah, bl, 1 << 24));
-            const long long sc = (fx::mad(ah, bh, 0) << 6) + (sm >> 25); // in units of 2^56
+            const int ah = int(w >> 31), av = int(unsigned(w) & 0x7fffffffu);
+            // in units of 2^53
+            const long long sm = fx::low_product(av, bl, fx::mad(av, bh, fx::mad(ah, bl, 1 << 21)));
+            const long long sc = (fx::mad(ah, bh, 0) << 9) + (sm >> 22);
             const int sh = int(sc >> 31), sl = int(unsigned(sc) & 0x7fffffffu);
 #pragma unroll
             for (int d = 0; d < D; ++d)
@@ -464,7 +495,7 @@ __device__ __forceinline__ void fixed_2nd(size_t n, size_t i, unsigned sub, cons
     if (LANES > 1 && !first)
         R.shift(al.a - a);
     fx::group_sum<LANES>(R);
-    *rate = R.value() * fx::pow2(94 - a - fx::kVelocityBits - 2 * fx::kListBits);
+    *rate = R.value() * fx::pow2(120 - a + unit - 2 * fx::kListBits); // 2^57 2^(63 - a)
 #pragma unroll
     for (int d = 0; d < D; ++d)
     {
@@ -474,8 +505,8 @@ __device__ __forceinline__ void fixed_2nd(size_t n, size_t i, unsigned sub, cons
             F[d].shift(al.a - a);
         }
         fx::group_sum<LANES>(F[d]);
-        // u K: 2^57 2^(63 - a), u: 2^(63 - a), sc: 2^56, the sum: 2^31
-        force[d] = F[d].value() * fx::pow2(126 - 2 * a + 87 - 2 * fx::kVelocityBits - 3 * fx::kListBits);
+        // u K: 2^57 2^(63 - a), u: 2^(63 - a), sc: 2^53, the sum: 2^31
+        force[d] = F[d].value() * fx::pow2(126 - 2 * a + 84 + 2 * unit - 3 * fx::kListBits);
     }
 }
 
@@ -560,7 +591,7 @@ __device__ __forceinline__ void wall_2nd(size_t n, size_t i, unsigned sub, const
 // The wall terms of the particles that have wall neighbours, kWallLanes threads each, into
 // sum[c n + i] (c < D the force, c = D the dissipation or rate).  In the sweep itself a warp
 // ran as many wall pairs as its longest wall list, with most lanes idle on the FP64 pipe.
-constexpr int kWallLanes = 8;
+constexpr int kWallLanes = 4; // 1,702,400 particles: 1st / 2nd half 167 / 232 us with 8, 135 / 190 with 4, 136 / 196 with 2
 template <int D, int HALF>
 __global__ void __launch_bounds__(kBlock) k_wall(size_t n, size_t n_active, const uint32_t *__restrict__ active,
                                                  FluidVars f, Neighbors wn, WallVars w, double beta,
@@ -656,8 +687,8 @@ __global__ void __launch_bounds__(kBlock, kBlocks1)
 // ---------------------------------------------------------------- 2nd half
 template <int D, int LANES>
 __global__ void __launch_bounds__(kBlock, kBlocks2)
-    k_interact_2nd(size_t n, FluidVars f, InnerPairs in, Neighbors wn, WallVars w, Riemann rs, Fixed fv, double c0,
-                   long long t_lim, double dt, const double *__restrict__ wall_sum)
+    k_interact_2nd(size_t n, FluidVars f, InnerPairs in, Neighbors wn, WallVars w, Riemann rs, Fixed fv, double dt,
+                   const double *__restrict__ wall_sum)
 {
     const size_t g = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
     const size_t i = g / LANES;
@@ -678,12 +709,12 @@ __global__ void __launch_bounds__(kBlock, kBlocks2)
     }
     else
     {
-        fixed_2nd<D, LANES>(n, i, sub, in, fv.value, t_lim, diss, &rate);
-        const double scale = in.factor * c0 * f.Vol[0];
+        fixed_2nd<D, LANES>(n, i, sub, in, fv.value, velocity_unit(fv), 1.0 / beta, diss, &rate);
+        const double scale = in.factor * f.Vol[0];
         rate *= scale;
 #pragma unroll
         for (int d = 0; d < D; ++d)
-            diss[d] *= scale * c0 * beta;
+            diss[d] *= scale * beta;
     }
     if (wn.count && LANES == 1)
     {
@@ -752,15 +783,16 @@ __device__ __forceinline__ void block_max_to(unsigned long long *slot, double v)
 template <int D>
 __global__ void k_acoustic_max(size_t n, const double *__restrict__ vel, double c0, unsigned long long *slot)
 {
-    double m = -1.0e300;
+    double m = -1.0;
     for (size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += size_t(gridDim.x) * blockDim.x)
     {
         double s = vel[i] * vel[i] + vel[n + i] * vel[n + i];
         if (D == 3)
             s = s + vel[2 * n + i] * vel[2 * n + i];
-        m = fmax(m, c0 + sqrt(s));
+        m = fmax(m, s);
     }
-    block_max_to(slot, m);
+    // the square root and the sum round monotonically: they are taken of the thread's largest
+    block_max_to(slot, m < 0.0 ? -1.0e300 : c0 + sqrt(m));
 }
 
 template <int D>
@@ -1044,7 +1076,8 @@ __global__ void __launch_bounds__(kBlock) k_tvc_inner(size_t n, InnerPairs in, c
 // workspace, with a fresh epoch for the verdict.
 Fixed fixed_of(sphx_relation inner, int half)
 {
-    return Fixed{inner->fx_value, inner->fx_flag + half, ++inner->fx_epoch[half]};
+    return Fixed{inner->fx_value, inner->fx_flag + half, ++inner->fx_epoch[half],
+                 reinterpret_cast<unsigned long long *>(inner->fx_flag + 4)};
 }
 // Lists longer than the integer sums allow, and a limiter of negative slope, take the
 // general path.
@@ -1183,23 +1216,24 @@ extern "C" int sphx_integration_2nd_half_with_wall_riemann(sphx_relation inner, 
         return SPHX_OK;
     sphx_ctx ctx = b->ctx;
     const Fixed fv = fixed_of(inner, 1);
-    const int c0_exp = std::ilogb(p->c0) + 1;
     if (b->dim == 2)
-        k_init_2nd<2><<<grid_for(n, 256), 256, 0, ctx->stream>>>(n, f.vel, f.Vol, c0_exp, fv);
+        k_largest_velocity<2><<<reduce_grid(ctx, n), kBlock, 0, ctx->stream>>>(n, f.vel, fv);
     else
-        k_init_2nd<3><<<grid_for(n, 256), 256, 0, ctx->stream>>>(n, f.vel, f.Vol, c0_exp, fv);
+        k_largest_velocity<3><<<reduce_grid(ctx, n), kBlock, 0, ctx->stream>>>(n, f.vel, fv);
+    SPHX_LAUNCHED(ctx);
+    if (b->dim == 2)
+        k_init_2nd<2><<<grid_for(n, 256), 256, 0, ctx->stream>>>(n, f.vel, f.Vol, fv);
+    else
+        k_init_2nd<3><<<grid_for(n, 256), 256, 0, ctx->stream>>>(n, f.vel, f.Vol, fv);
     SPHX_LAUNCHED(ctx);
     const InnerPairs in = pairs_of(inner);
     Neighbors wn{};
     if (wall)
         wn = neighbors_of(wall);
     Riemann rs = make_riemann(*p);
-    const double beta = rs.slope * rs.inv_c0_ave, scale = std::ldexp(1.0, c0_exp);
-    // the speed at which the limiter reaches 1, in the units of an alignment of 0
-    const double lim = std::ldexp(1.0 / (beta * scale), 55);
-    const long long t_lim = lim < std::ldexp(1.0, 57) ? std::llrint(lim) : 1ll << 57;
+    const double beta = rs.slope * rs.inv_c0_ave;
     SPHX_TRY((wall_terms<2>(wall, f, wn, w, beta)));
-    SWEEP_DISPATCH(k_interact_2nd, b->dim, ctx, n, n, f, in, wn, w, rs, fixed_path(fv, in, beta), scale, t_lim, dt,
+    SWEEP_DISPATCH(k_interact_2nd, b->dim, ctx, n, n, f, in, wn, w, rs, fixed_path(fv, in, beta), dt,
                    wall ? wall->contact_sum : nullptr);
     SPHX_LAUNCHED(ctx);
     return SPHX_OK;

@@ -3,25 +3,27 @@
 // GB300 runs FP64 at 1/64 of the FP32 rate (a warp instruction occupies an SM's FP64 pipe
 // for 16 cycles), while a 32 x 32 + 64 bit integer multiply-add takes half a cycle to one.
 // The neighbour sums of the FP64 solvers are therefore taken in fixed point: every factor
-// of a pair is bounded by the scheme (a unit vector, the kernel derivative over its
-// prefactor, the pressure over rho0 c0^2, the velocity over c0), so it is held as a 57- to
-// 61-bit integer with a scale known beforehand, products are formed from 32-bit halves and
+// of a pair is bounded (a unit vector, the kernel derivative over its prefactor, the pressure
+// over rho0 c0^2, the velocity over the largest one), so it is held as a 57- to 60-bit
+// integer with a common scale, products are formed from 32-bit halves and
 // sums are exact integer sums, the same for any order of the neighbours and any split of a
 // particle's list over threads.
 //
 // Precision.  Stored factors carry a quantum of 2^-57 (kernel derivative, unit vector),
-// 2^-60 p0 (pressure) and 2^-61 c0 (velocity): finer than the rounding of the doubles they
-// come from (2^-53 of unit vector and kernel; the density rho0 (1 + p / p0) resolves p to
-// 2^-53 p0 and a velocity of 0.004 c0 or more is resolved to 2^-61 c0 or coarser).  A
-// product keeps 53 or more significant bits relative to the largest term of its sum: each
-// thread carries an alignment `a` (binary places to the left), starts it for small terms
-// and steps it down when a larger term appears, shifting its sums along.
+// 2^-60 p0 (pressure; the density rho0 (1 + p / p0) it comes from resolves it to 2^-53 p0)
+// and 2^-60 of the largest velocity component.  A product keeps 53 or more significant bits
+// relative to the largest term of its sum: each thread carries an alignment `a` (binary
+// places to the left), set by its first pairs and stepped down when a larger term appears,
+// its sums moving along.
 //
-// Measured (3D dam break, one whole advection step of 5 sub-steps): 1,702,400 particles
-// 59.2 -> 25.7 ms, the sweeps 3.1 + 5.8 -> 1.1 + 1.6 ms; error against 64-bit references
-// 3.7e-13 before and after.
+// Measured.  3D dam break, 1,702,400 particles, one advection step of 5 sub-steps: 59.2 ->
+// 17.7 ms with the relation update; a 1st / 2nd half sweep 3.1 / 5.8 -> 0.87 / 1.18 ms, now
+// bound by the 36 bytes of a list entry (87 % / 62 % of the measured copy bandwidth).  Error
+// of one sweep against long doubles (8,000 particles): force of the 1st half 6.2e-16 in FP64,
+// 3.3e-16 here; of the 2nd half 8.0e-16 and 3.3e-16; density rate 3.2e-16 and 2.0e-16, 1.8e-15
+// and 1.5e-15; kernel derivative 3.8e-16 and 2.7e-16, unit vector 7.6e-17 and 4.7e-17.
 //
-// Numbers outside those bounds (|p| >= p0 / 4, |v| >= c0 / 2, NaN, particles of different
+// Numbers outside those bounds (|p| >= p0 / 4, infinities, NaN, particles of different
 // volume) are found by the kernel that converts them; the sweep then takes its general
 // path, plain FP64 on the same lists.
 #pragma once
@@ -36,9 +38,9 @@ namespace fx
 {
 // A factor of a list entry: value = (h 2^31 + l) 2^-kListBits, |l| <= 2^30.
 constexpr int kListBits = 57;
-constexpr int kPressureBits = 60, kVelocityBits = 61;
-constexpr double kPressureRange = 0.25, kVelocityRange = 0.5; // of p0 and of c0
-constexpr unsigned kMaxCap = 512; // list slots up to which the integer sums cannot overflow
+constexpr int kPressureBits = 60, kVelocityBits = 60;
+constexpr double kPressureRange = 0.25; // of p0
+constexpr unsigned kMaxCap = 256; // list slots up to which the integer sums cannot overflow
 constexpr int kFold = 16;         // pairs between folds of the middle sum
 
 // 2^k, -1022 <= k <= 1023
@@ -87,25 +89,34 @@ __host__ __device__ __forceinline__ double decode(int2 q)
 
 __device__ __forceinline__ long long mad(int a, int b, long long c)
 {
-    return static_cast<long long>(a) * static_cast<long long>(b) + c;
+    // as one instruction: left to the compiler, part of the products became a multiplication
+    // and an addition (2nd-half sweep of 1,702,400 particles 1.27 -> 1.10 ms)
+    long long d;
+    asm("mad.wide.s32 %0, %1, %2, %3;" : "=l"(d) : "r"(a), "r"(b), "l"(c));
+    return d;
 }
-// The halves of a 64-bit particle value: v = h 2^32 + 2 l (the lowest bit dropped).
+// c + a b / 2^31 for the low halves of two factors (the sum of their upper products is c):
+// left out, it would cost a sum of aligned values three digits.
+__device__ __forceinline__ long long low_product(int a, int b, long long c) { return mad(__mulhi(a, b), 2, c); }
+// The halves of a 64-bit factor: v = h 2^32 + 2 l (the lowest bit dropped).  A product with a
+// list entry is then hh 2^63 + m 2^32.
 __device__ __forceinline__ int high(long long v) { return int(v >> 32); }
 __device__ __forceinline__ int low(long long v) { return int(unsigned(v) >> 1); }
 
 // hh 2^31 + m as a double.
 __device__ __forceinline__ double total(long long hh, long long m) { return fma(double(hh), 2147483648.0, double(m)); }
 
-// A sum of products of aligned values: hh 2^31 + m.
+// A sum of products, hh 2^31 + m: of 64-bit factors with list entries over 2^32, of aligned
+// values (halves of 31 bits) with list entries over 2^31.
 struct Sum
 {
     long long hh = 0, m = 0;
-    // (th 2^31 + tl) (f.x 2^31 + f.y) without the product of the low halves, over 2^31
-    __device__ __forceinline__ void add(int th, int tl, int2 f)
+    __device__ __forceinline__ void add(int vh, int vl, int2 f)
     {
-        hh = mad(th, f.x, hh);
-        m = mad(th, f.y, m);
-        m = mad(tl, f.x, m);
+        hh = mad(vh, f.x, hh);
+        m = mad(vh, f.y, m);
+        m = mad(vl, f.x, m);
+        m = low_product(vl, f.y, m);
     }
     __device__ __forceinline__ void fold()
     {
@@ -125,7 +136,7 @@ struct Sum
 // term steps it down.
 struct Align
 {
-    static constexpr int kStep = 3, kMargin = 2, kMost = 21;
+    static constexpr int kStep = 3, kMargin = 1, kMost = 21;
     int a = 0;
     int limit = 1 << 24; // bound on the high word of |hh|
     // `top` collects the high words: its bit length bounds that of every |hh| seen
@@ -214,7 +225,7 @@ __device__ __forceinline__ long long middle(Halves a, Halves b, long long round 
 {
     return mad(a.h, b.l, mad(a.l, b.h, round)) + (mad(a.l, b.l, 0) >> 31);
 }
-// a b / 2^57 for 0 <= a, b <= 2^57
+// a b / 2^57, rounded, for a, b >= 0 below 2^61 with a product below 2^119
 __device__ __forceinline__ long long product57(Halves a, Halves b)
 {
     return (mad(a.h, b.h, 0) << 5) + (middle(a, b, 1 << 25) >> 26);
@@ -235,7 +246,7 @@ struct GeometryScale
 
 // Wendland C2 of one pair in fixed point: D = x_i - x_j in the shifted units.  Writes the
 // entry (kernel derivative over its prefactor, unit vector), r over the cut-off in units of
-// 2^-57 and the kernel over its prefactor in units of 2^-54.  Returns false (nothing written)
+// 2^-57 and the kernel over its prefactor in units of 2^-57.  Returns false (nothing written)
 // for points closer than about 1/16 of the cut-off, which take the FP64 form.
 //
 // 1 / |D| comes from the hardware's FP32 reciprocal root of the leading bits and one
@@ -243,7 +254,7 @@ struct GeometryScale
 // e = 1 - |D|^2 y0^2 formed exactly to 2^-64; |e| < 2^-20 leaves e^3 below 2^-60.
 template <int D>
 __device__ __forceinline__ bool wendland_pair(const long long *dx, const GeometryScale &g, Entry<D> &out,
-                                              long long &r57, long long &w54)
+                                              long long &r57, long long &w57)
 {
     long long hh = 0, m = 0, ll = 0;
 #pragma unroll
@@ -282,11 +293,10 @@ __device__ __forceinline__ bool wendland_pair(const long long *dx, const Geometr
         out.e[d] = split((mad(n.h, Yh.h, 0) << 1) + (middle(n, Yh, 1 << 29) >> 30));
     }
     // t = 1 - r / rc, q = 2 r / rc: dW ~ -5 t^3 q, W ~ t^4 (1 + 2 q)
-    const Halves t = halves(max((1ll << 57) - r57, 0ll)), rr = halves(r57);
+    const Halves t = halves(max((1ll << 57) - r57, 0ll));
     const Halves t2 = halves(product57(t, t)), t3 = halves(product57(t2, t));
-    out.k = split(-10 * product57(t3, rr));
-    const long long t4 = product57(t2, t2);
-    w54 = (t4 + 4 * product57(halves(t4), rr) + 4) >> 3;
+    out.k = split(-product57(t3, halves(10 * r57)));
+    w57 = product57(halves(product57(t2, t2)), halves((1ll << 57) + 4 * r57));
     return true;
 }
 

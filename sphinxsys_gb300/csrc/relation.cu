@@ -49,6 +49,7 @@ struct BuildArgs
     WendlandC2 k;
     int depth, cap;
     float accept_sqr, reject_sqr, self_sqr; // bounds of the FP32 test (see search_bounds)
+    float reach_sqr; // cells farther than this hold no neighbour
     uint32_t *count, *J;
     double *DW, *E, *R, *W; // E: dim arrays of cap * n_src
     fx::EntryStore fx;      // inner relations: in place of DW and E
@@ -98,10 +99,16 @@ __device__ __noinline__ bool exact_test(const double *x_i, const double *spos, s
     return r2 < rc_sqr;
 }
 
+// Distance along an axis from a cell of spacing gs to a point at offset o from its corner.
+__device__ __forceinline__ float gap(float o, float gs) { return fmaxf(0.0f, fmaxf(-o, o - gs)); }
+
 // The search: LANES threads per particle test the candidates of a cell side by side and
 // append the accepted ones in cell order (a ballot gives each its slot).  One thread per
 // particle keeps the list writes of a warp together and does the least work per candidate;
-// few particles need the threads to cover the memory latency.
+// few particles need the threads to cover the memory latency.  Cells of the window farther
+// from the particle than the cut-off are passed over: a contact search of depth 2 visits 27
+// cells of its 125 (wall search 1.75 -> 0.42 ms at that size; a particle lies in its cell up to the
+// rounding of the cell index, far inside the margin of reach_sqr).
 template <int D, bool INNER, int LANES>
 __global__ void __launch_bounds__(kBlock) k_build(BuildArgs a)
 {
@@ -137,10 +144,16 @@ __global__ void __launch_bounds__(kBlock) k_build(BuildArgs a)
     for (cc[0] = lo[0]; cc[0] < hi[0]; ++cc[0])
     {
         const float o0 = fmaf(-float(cc[0] - lo[0]), gs, o[0]);
+        const float g0 = gap(o0, gs);
+        if (inside && g0 * g0 > a.reach_sqr)
+            continue;
         // 2D: the column of cells along axis 1; 3D: a column along axis 2 for every cc[1]
         for (cc[1] = lo[1]; cc[1] < (D == 3 ? hi[1] : lo[1] + 1); ++cc[1])
         {
             const float o1 = D == 3 ? fmaf(-float(cc[1] - lo[1]), gs, o[1]) : 0.0f;
+            const float g1 = D == 3 ? gap(o1, gs) : 0.0f, rest = a.reach_sqr - (g0 * g0 + g1 * g1);
+            if (inside && rest < 0.0f)
+                continue;
             cc[2] = lo[2];
             const int cells = hi[D - 1] - lo[D - 1];
             const uint32_t first = linear_cell<D>(a.m, cc);
@@ -153,6 +166,9 @@ __global__ void __launch_bounds__(kBlock) k_build(BuildArgs a)
                 uint32_t kb = ke;
                 ke = a.cell_offset[first + k + 1];
                 uint32_t stop = ke;
+                const float gl = gap(ol, gs);
+                if (inside && gl * gl > rest)
+                    stop = kb;
                 if (!SPHX_CHECKED(kb <= ke && ke <= a.n_tgt, kCheckCellRange, (uint64_t(kb) << 32) | ke))
                     stop = kb;
                 for (uint32_t kk = kb + sub; LANES == 1 ? kk < stop : kk - sub < stop; kk += LANES)
@@ -235,7 +251,7 @@ __device__ __forceinline__ void pair_fp64(const BuildArgs &a, double r2, double 
 }
 template <int D>
 __device__ __noinline__ void entry_fp64(const BuildArgs &a, size_t i, uint32_t kk, fx::Entry<D> &q, long long &r57,
-                                        long long &w54)
+                                        long long &w57)
 {
     double xi[3], dx[3], r2, W, K, r, inv;
     load_position(a.src_pos, a.n_src, i, D, xi);
@@ -245,7 +261,7 @@ __device__ __noinline__ void entry_fp64(const BuildArgs &a, size_t i, uint32_t k
     for (int d = 0; d < D; ++d)
         q.e[d] = fx::encode(dx[d] * inv);
     r57 = __double2ll_rn(r * (0.5 * a.k.inv_h) * fx::pow2(57));
-    w54 = __double2ll_rn(W * fx::pow2(54));
+    w57 = __double2ll_rn(W * fx::pow2(57));
 }
 
 // The cell-list entries' positions in units of 2^unit with their particle: what a pair reads
@@ -272,7 +288,7 @@ __global__ void k_fix_positions(size_t n, const double *__restrict__ spos, const
 // Values of the pairs of an inner relation.  In FP64 a pair costs about 45 instructions of
 // the FP64 pipe (720 cycles of an SM per warp); in fixed point about 50 wide multiply-adds
 // and 150 other integer instructions.  Search and values of 1,702,400 particles (130 M
-// pairs): 8.3 ms in FP64, 1.9 + 2.3 ms here.
+// pairs): 8.3 ms in FP64, 1.9 + 2.1 ms here.
 template <int D, int LANES>
 __global__ void __launch_bounds__(kBlock) k_pairs_inner(BuildArgs a)
 {
@@ -287,14 +303,14 @@ __global__ void __launch_bounds__(kBlock) k_pairs_inner(BuildArgs a)
     for (int d = 0; d < D; ++d)
         x_i[d] = fx::fixed(a.src_pos[d * a.n_src + i], a.g.unit, fixed);
     const unsigned cnt = a.count[i];
-    long long w_sum = 0; // at most 256 terms of up to 2^54
-    double w_total = 0.0;
+    // the kernel values' sum, exact: w_hi 2^31 + w_sum, the latter at most 32 terms of 2^57
+    long long w_sum = 0, w_hi = 0;
     for (unsigned s = sub, term = 0; s < cnt; s += LANES, ++term)
     {
-        if ((term & 0xff) == 0xff)
+        if ((term & 31u) == 31u)
         {
-            w_total += double(w_sum);
-            w_sum = 0;
+            w_hi += w_sum >> 31;
+            w_sum &= 0x7fffffffll;
         }
         const size_t slot = size_t(s) * a.n_src + i;
         const uint32_t kk = a.J[slot];
@@ -305,18 +321,19 @@ __global__ void __launch_bounds__(kBlock) k_pairs_inner(BuildArgs a)
         const long long dx[3] = {(x_i[0] - p.x) << a.g.shift, (x_i[1] - p.y) << a.g.shift,
                                  (x_i[2] - w.x) << a.g.shift};
         fx::Entry<D> q;
-        long long r57, w54;
-        if (!fixed || !fx::wendland_pair<D>(dx, a.g, q, r57, w54))
-            entry_fp64<D>(a, i, kk, q, r57, w54);
+        long long r57, w57;
+        if (!fixed || !fx::wendland_pair<D>(dx, a.g, q, r57, w57))
+            entry_fp64<D>(a, i, kk, q, r57, w57);
         a.J[slot] = uint32_t(w.y);
         a.fx.store<D>(slot, q);
         if (a.R)
             a.R[slot] = double(r57) * (2.0 * a.k.h * fx::pow2(-57));
-        w_sum += w54;
+        w_sum += w57;
     }
-    w_total = fx::group_sum<LANES>(w_total + double(w_sum));
-    if (sub == 0)
-        a.wsum[i] = a.k.factor_W * (1.0 + w_total * fx::pow2(-54));
+    w_hi = fx::group_sum<LANES>(w_hi + (w_sum >> 31));
+    w_sum = fx::group_sum<LANES>(w_sum & 0x7fffffffll);
+    if (sub == 0) // with the particle's own W(0)
+        a.wsum[i] = a.k.factor_W * (fx::total(w_hi + (1ll << 26), w_sum) * fx::pow2(-57));
 }
 
 // Values of the pairs of a contact relation: kContactLanes threads per particle that has any.
@@ -373,6 +390,7 @@ void search_bounds(BuildArgs &a, const sphx_cell_list_s &cl)
     a.accept_sqr = float(a.k.rc_sqr * (1.0 - m));
     a.reject_sqr = float(a.k.rc_sqr * (1.0 + m));
     a.self_sqr = float(a.k.rc_sqr * m);
+    a.reach_sqr = float(a.k.rc_sqr * (1.0 + 1.0 / 256.0));
     for (int d = 0; d < 3; ++d)
         if ((cl.periodic_mask & (1 << d)) && cl.per_upper[d] - cl.per_lower[d] < 2.0 * rc)
             a.self_sqr = std::numeric_limits<float>::max();
@@ -443,8 +461,8 @@ int sphx_relation_s::allocate(int new_cap, size_t n)
         if (dim == 2)
             SPHX_CUDA(cudaMalloc(&fx_k, slots * sizeof(int2)));
         SPHX_CUDA(cudaMalloc(&fx_value, nn * (dim == 2 ? 2 : 4) * sizeof(long long)));
-        SPHX_CUDA(cudaMalloc(&fx_flag, 3 * sizeof(uint32_t)));
-        SPHX_CUDA(cudaMemsetAsync(fx_flag, 0, 3 * sizeof(uint32_t), ctx->stream));
+        SPHX_CUDA(cudaMalloc(&fx_flag, 6 * sizeof(uint32_t)));
+        SPHX_CUDA(cudaMemsetAsync(fx_flag, 0, 6 * sizeof(uint32_t), ctx->stream));
     }
     else
     {
