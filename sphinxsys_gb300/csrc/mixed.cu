@@ -205,6 +205,17 @@ __global__ void SPHX_BUILD_BOUNDS k_mp_build(size_t n, MPConst k, MPFluid f, con
                           max_counts);
 }
 
+template <int D, int L>
+__global__ void __launch_bounds__(256) k_mp_build_lanes(size_t n, MPConst k, MPFluid f,
+                                                        const uint32_t *__restrict__ f_offset, MPWall w,
+                                                        const uint32_t *__restrict__ w_offset, MPLists in, MPLists wl,
+                                                        unsigned int *max_counts)
+{
+    const size_t t = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
+    if (t / L < n) // whole groups
+        build_particle_lanes<D, L>(t / L, n, k.p, Visit{k.m, 0u, f_offset, w_offset}, f, w, in, wl, max_counts);
+}
+
 // Tile key of every particle (cell order) for the tile-grouped traversal order.
 template <int D>
 __global__ void k_mp_tile_key(size_t n, const float4 *__restrict__ geo0, TileShape ts, uint32_t *__restrict__ key,
@@ -253,6 +264,86 @@ __global__ void k_mp_density(size_t n, const float *__restrict__ drho_sum, float
 }
 
 // ---------------------------------------------------------------- acoustic sub-step
+// The sub-steps of an advection step without a host round trip each: the step sizes and the
+// relaxation time before every sub-step live in a device record, formed by the sub-step's
+// first kernel from the acoustic maximum of the one before (the host's expressions and
+// rounding).  Sub-steps enqueued past the end of the relaxation see it there and do nothing.
+// Waiting for every maximum cost a coarse run most of its step (5,000 particles: 375 us).
+constexpr int kRecordSteps = 32; // sub-steps enqueued between two looks at the record
+struct StepRecord
+{
+    double relax[kRecordSteps], dt[kRecordSteps];
+    unsigned long long ac[2]; // acoustic maximum after sub-step s in ac[(s + 1) & 1]
+};
+struct StepPlan
+{
+    StepRecord *rec;
+    unsigned long long *slots;
+    double Dt, cfl_h, relax0, first_dt; // first_dt: of loop style 1
+    int style, periodic;
+};
+// Sub-step s of a plan: its size, and whether the relaxation was still short of Dt.
+struct StepArg
+{
+    const StepRecord *rec;
+    double Dt;
+    int s;
+};
+__device__ __forceinline__ bool step_active(double) { return true; }
+__device__ __forceinline__ bool step_active(const StepArg &a) { return a.rec->relax[a.s] < a.Dt; }
+__device__ __forceinline__ double step_size(const StepArg &a) { return a.rec->dt[a.s]; }
+
+// One thread of a block forms the step size (FP64, with a division) for its kInitItems
+// particles a thread.
+constexpr int kInitItems = 4;
+__global__ void __launch_bounds__(256) k_mp_init1_planned(size_t n, float *__restrict__ drho,
+                                                          const float *__restrict__ drho_dt, float4 *__restrict__ dyn,
+                                                          float *__restrict__ pres, float p0_over_rho0, StepPlan pl,
+                                                          int s)
+{
+    __shared__ float half_dt;
+    __shared__ bool active;
+    if (threadIdx.x == 0)
+    {
+        StepRecord *r = pl.rec;
+        // what is read here was written by earlier kernels; this one writes the entries of s
+        const double ac = from_ordered_bits(s == 0 ? pl.slots[0] : r->ac[s & 1]);
+        double dt = pl.cfl_h / (ac + kTinyReal);
+        if (pl.style == 0)
+            dt = pl.periodic ? fmin(dt, pl.Dt) : dt; // dt = SMIN(acoustic dt, Dt) (taylor_green.cpp:146)
+        else if (s == 0)
+            dt = pl.first_dt;
+        const double relax = s == 0 ? pl.relax0 : r->relax[s - 1] + (pl.style == 0 ? r->dt[s - 1] : dt);
+        active = relax < pl.Dt;
+        half_dt = float(0.5 * dt);
+        if (blockIdx.x == 0)
+        {
+            r->dt[s] = dt;
+            r->relax[s] = relax;
+            if (relax < pl.Dt)
+            {
+                r->ac[(s + 1) & 1] = 0;
+                pl.slots[1] = 0;
+            }
+        }
+    }
+    __syncthreads();
+    if (!active)
+        return;
+#pragma unroll
+    for (int q = 0; q < kInitItems; ++q)
+    {
+        const size_t i = (size_t(blockIdx.x) * kInitItems + q) * blockDim.x + threadIdx.x;
+        if (i >= n)
+            break;
+        const float d = drho[i] + drho_dt[i] * half_dt;
+        drho[i] = d;
+        const float p = p0_over_rho0 * d;
+        reinterpret_cast<float *>(dyn)[4 * i + 3] = p;
+        pres[i] = p;
+    }
+}
+
 __global__ void k_mp_init1(size_t n, float *__restrict__ drho, const float *__restrict__ drho_dt,
                            float4 *__restrict__ dyn, float *__restrict__ pres, float p0_over_rho0, float half_dt)
 {
@@ -611,9 +702,40 @@ __global__ void k_mp_second_lanes(size_t n, MPConst k, MPFluid f, MPWall w, MPLi
     warp_max_to(adv_slot, amax);
 }
 
+// The stored-list sweeps with L lanes per particle and the sums of strategy 0.
+template <int D, int L, class Step>
+__global__ void __launch_bounds__(256) k_mp_first_ordered(size_t n, MPConst k, MPFluid f, MPWall w, MPLists in,
+                                                          MPLists wl, Step step, unsigned long long *ac_slot)
+{
+    if (!step_active(step))
+        return;
+    const size_t t = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
+    double vmax = -1.0e300;
+    if (t / L < n)
+        vmax = first_particle<D, true, 0, L, true>(t / L, n, k.p, Visit{k.m, 0u, nullptr, nullptr}, step, f, w, in, wl);
+    warp_max_to(ac_slot, vmax);
+}
+template <int D, int L, class Step>
+__global__ void __launch_bounds__(256) k_mp_second_ordered(size_t n, MPConst k, MPFluid f, MPWall w, MPLists in,
+                                                           MPLists wl, Step step, unsigned long long *adv_slot)
+{
+    if (!step_active(step))
+        return;
+    const size_t t = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
+    double amax = -1.0e300;
+    if (t / L < n)
+        amax = second_particle<D, true, 0, L, true>(t / L, n, k.p, Visit{k.m, 0u, nullptr, nullptr}, step, f, w, in, wl);
+    warp_max_to(adv_slot, amax);
+}
 // Lanes per particle of strategies 5 and 6 (0 for the others).
 inline int strategy_lanes(int strategy) { return strategy == 5 ? 2 : (strategy == 6 ? 4 : 0); }
 
+// Particles per SM up to which 8 lanes share a particle, with the bits of one: the 3D sweeps
+// and the configuration build.  One step, 3D dam break of 11,200 particles (74 per SM): 587 us
+// with neither, 515 with the build, 435 with both; 26,720 (176 per SM): 585, 555, 555 without
+// the sweeps and 594 with them; 46,000 (303 per SM): 617, 617.  2D sweeps, periodic sweeps and
+// 2 or 4 lanes gained nothing at any size.
+constexpr size_t kLanesSweep = 100, kLanesBuild = 200;
 // Blocks of 256 threads per SM the stored-list / cell sweeps are compiled to fit (the
 // register cap follows: 4 -> 64, 5 -> 48 registers; 0 leaves the 2nd half unbounded: with
 // the packed x / y arithmetic it would take 66): build-time tuning parameters.
@@ -646,41 +768,47 @@ inline int strategy_lanes(int strategy) { return strategy == 5 ? 2 : (strategy =
 #define SPHX_SECOND_ATTR SPHX_SECOND_BOUNDS
 #endif
 
-template <int D, bool LISTS, bool ORDER>
+template <int D, bool LISTS, bool ORDER, class Step>
 __global__ void SPHX_FIRST_ATTR k_mp_first(size_t n, MPConst k, MPFluid f, const uint32_t *__restrict__ f_offset, MPWall w,
-               const uint32_t *__restrict__ w_offset, MPLists in, MPLists wl, double dt,
+               const uint32_t *__restrict__ w_offset, MPLists in, MPLists wl, Step step,
                unsigned long long *ac_slot, const uint32_t *__restrict__ order)
 {
+    if (!step_active(step))
+        return;
     size_t t = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
     double vmax = -1.0e300;
     if (t < n)
-        vmax = first_particle<D, LISTS>(particle_of<ORDER>(t, order), n, k.p, Visit{k.m, 0u, f_offset, w_offset}, dt,
+        vmax = first_particle<D, LISTS>(particle_of<ORDER>(t, order), n, k.p, Visit{k.m, 0u, f_offset, w_offset}, step,
                                         f, w, in, wl);
     warp_max_to(ac_slot, vmax);
 }
 
-template <int D, bool LISTS, bool ORDER>
+template <int D, bool LISTS, bool ORDER, class Step>
 __global__ void SPHX_SECOND_ATTR k_mp_second(size_t n, MPConst k, MPFluid f, const uint32_t *__restrict__ f_offset, MPWall w,
-                const uint32_t *__restrict__ w_offset, MPLists in, MPLists wl, double dt,
+                const uint32_t *__restrict__ w_offset, MPLists in, MPLists wl, Step step,
                 unsigned long long *adv_slot, const uint32_t *__restrict__ order)
 {
+    if (!step_active(step))
+        return;
     size_t t = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
     double amax = -1.0e300;
     if (t < n)
         amax = second_particle<D, LISTS>(particle_of<ORDER>(t, order), n, k.p, Visit{k.m, 0u, f_offset, w_offset},
-                                         dt, f, w, in, wl);
+                                         step, f, w, in, wl);
     warp_max_to(adv_slot, amax);
 }
 
-template <int D, bool LISTS>
+template <int D, bool LISTS, class Step>
 __global__ void __launch_bounds__(256, 4) k_mp_first_periodic(size_t n, MPConst k, MPFluid f,
                                                                const uint32_t *__restrict__ f_offset, MPLists in,
-                                                               double dt, unsigned long long *ac_slot)
+                                                               Step step, unsigned long long *ac_slot)
 {
+    if (!step_active(step))
+        return;
     size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
     double vmax = -1.0e300;
     if (i < n)
-        vmax = first_particle_periodic<D, LISTS>(i, n, k.p, k.m, f_offset, dt, f, in);
+        vmax = first_particle_periodic<D, LISTS>(i, n, k.p, k.m, f_offset, step, f, in);
     warp_max_to(ac_slot, vmax);
 }
 
@@ -695,14 +823,16 @@ __global__ void __launch_bounds__(256, 4) k_mp_first_periodic(size_t n, MPConst 
 #define SPHX_PERIODIC_SECOND_BOUNDS
 #endif
 
-template <int D, bool LISTS, bool RIEMANN>
+template <int D, bool LISTS, bool RIEMANN, class Step>
 __global__ void SPHX_PERIODIC_SECOND_BOUNDS k_mp_second_periodic(size_t n, MPConst k, MPFluid f, const uint32_t *__restrict__ f_offset,
-                                     MPLists in, double dt, unsigned long long *adv_slot)
+                                     MPLists in, Step step, unsigned long long *adv_slot)
 {
+    if (!step_active(step))
+        return;
     size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
     double amax = -1.0e300;
     if (i < n)
-        amax = second_particle_periodic<D, LISTS, RIEMANN>(i, n, k.p, k.m, f_offset, dt, f, in);
+        amax = second_particle_periodic<D, LISTS, RIEMANN>(i, n, k.p, k.m, f_offset, step, f, in);
     warp_max_to(adv_slot, amax);
 }
 
@@ -1005,6 +1135,8 @@ T *dalloc(size_t n)
 }
 } // namespace
 
+constexpr size_t kSlots = 12, kRecordWords = sizeof(StepRecord) / sizeof(unsigned long long);
+
 // Chunks of the position rows sphx_mp_upload_host copies and hashes in a pipeline.
 constexpr int kUploadChunks = 4;
 
@@ -1023,8 +1155,9 @@ struct sphx_mp_s
     // device scalars: 0 acoustic max, 1 advection max, 2 misc, 3 build counts, 4-5 state
     // check, 6-7 tile preparation (window maxima, tile count, build overflow), 8 sweep
     // overflow of the tiled strategy, 10-11 chunk counters of the persistent sweeps
-    unsigned long long *slots = nullptr;
+    unsigned long long *slots = nullptr; // kSlots scalars, then a StepRecord
     unsigned long long *h_slots = nullptr;
+    bool slots_read = false; // h_slots[0] and [1] hold the device's maxima
     double physical_time = 0, acoustic_dt = 0;
     // positions moved since the last configuration update: the re-hash, re-sort and list
     // build run at the start of the next advection step, so that a caller who replaces
@@ -1073,8 +1206,8 @@ namespace
 {
 // The periodic 2nd half with or without the Riemann dissipation (limiter slope 0 is the
 // reference's NoRiemannSolver).
-template <int D, bool LISTS>
-void launch_second_periodic(sphx_mp_s *mp, unsigned blk, double dt)
+template <int D, bool LISTS, class Step>
+void launch_second_periodic(sphx_mp_s *mp, unsigned blk, const Step &dt)
 {
     const size_t n = mp->n;
     cudaStream_t s = mp->ctx->stream;
@@ -1242,6 +1375,15 @@ int tile_prepare(sphx_mp mp)
     return SPHX_OK;
 }
 
+// Lanes per particle of the stored-list sweeps in cell order (1: one thread each).
+constexpr int kOrderedLanes = 8;
+int ordered_lanes(sphx_mp mp)
+{
+    if (mp->strategy != 0 || mp->order_active || mp->k.periodic || mp->dim == 2)
+        return 1;
+    return mp->n < size_t(std::max(1, mp->ctx->num_sms)) * kLanesSweep ? kOrderedLanes : 1;
+}
+
 template <int D>
 int launch_build(sphx_mp mp)
 {
@@ -1269,14 +1411,17 @@ int launch_build(sphx_mp mp)
         else if (mp->order_active)
             k_mp_build<D, true><<<grid_for(mp->n, 256), 256, 0, s>>>(mp->n, mp->k, mp->a, mp->f_offset, mp->w,
                                                                     mp->w_offset, mp->in, mp->wl, mc, mp->order);
+        else if (mp->n < size_t(std::max(1, ctx->num_sms)) * kLanesBuild)
+            k_mp_build_lanes<D, kOrderedLanes><<<grid_for(kOrderedLanes * mp->n, 256), 256, 0, s>>>(mp->n, mp->k, mp->a, mp->f_offset, mp->w,
+                                                                           mp->w_offset, mp->in, mp->wl, mc);
         else
             k_mp_build<D, false><<<grid_for(mp->n, 256), 256, 0, s>>>(mp->n, mp->k, mp->a, mp->f_offset, mp->w,
                                                                      mp->w_offset, mp->in, mp->wl, mc, nullptr);
         SPHX_LAUNCHED(ctx);
-        SPHX_CUDA(cudaMemcpyAsync(mp->h_slots + 3, mc, 2 * sizeof(unsigned int), cudaMemcpyDeviceToHost, s));
-        SPHX_CUDA(cudaMemcpyAsync(mp->h_slots + 7, mp->slots + 7, sizeof(unsigned long long), cudaMemcpyDeviceToHost,
+        SPHX_CUDA(cudaMemcpyAsync(mp->h_slots, mp->slots, kSlots * sizeof(unsigned long long), cudaMemcpyDeviceToHost,
                                   s));
         SPHX_CUDA(cudaStreamSynchronize(s));
+        mp->slots_read = true;
         if (mp->lists_tiled && reinterpret_cast<const unsigned int *>(mp->h_slots + 7)[1] != 0)
             return fail(SPHX_ERR_CAPACITY, "a tile window exceeded its staged capacity");
         const unsigned int *h = reinterpret_cast<const unsigned int *>(mp->h_slots + 3);
@@ -1349,19 +1494,19 @@ int settle_configuration(sphx_mp mp)
     return SPHX_OK;
 }
 
-template <int D, bool LISTS, bool ORDER>
-void launch_first(sphx_mp mp, unsigned blk, double dt)
+template <int D, bool LISTS, bool ORDER, class Step>
+void launch_first(sphx_mp mp, unsigned blk, const Step &dt, unsigned long long *ac)
 {
     const size_t n = mp->n;
-    k_mp_first<D, LISTS, ORDER><<<grid_for(n, blk), blk, 0, mp->ctx->stream>>>(
-        n, mp->k, mp->a, mp->f_offset, mp->w, mp->w_offset, mp->in, mp->wl, dt, mp->slots, mp->order);
+    k_mp_first<D, LISTS, ORDER, Step><<<grid_for(n, blk), blk, 0, mp->ctx->stream>>>(
+        n, mp->k, mp->a, mp->f_offset, mp->w, mp->w_offset, mp->in, mp->wl, dt, ac, mp->order);
 }
 
-template <int D, bool LISTS, bool ORDER>
-void launch_second(sphx_mp mp, unsigned blk, double dt)
+template <int D, bool LISTS, bool ORDER, class Step>
+void launch_second(sphx_mp mp, unsigned blk, const Step &dt)
 {
     const size_t n = mp->n;
-    k_mp_second<D, LISTS, ORDER><<<grid_for(n, blk), blk, 0, mp->ctx->stream>>>(
+    k_mp_second<D, LISTS, ORDER, Step><<<grid_for(n, blk), blk, 0, mp->ctx->stream>>>(
         n, mp->k, mp->a, mp->f_offset, mp->w, mp->w_offset, mp->in, mp->wl, dt, mp->slots + 1, mp->order);
 }
 
@@ -1498,6 +1643,127 @@ int deliver_rows(sphx_mp mp, int rows)
     return SPHX_OK;
 }
 
+// The 1st / 2nd half of the stored-list and cell strategies (0 and 1): the step size by value
+// or from the record, the acoustic maximum into *ac.
+template <int D, class Step>
+void sweep_first(sphx_mp mp, unsigned blk, const Step &step, unsigned long long *ac)
+{
+    const size_t n = mp->n;
+    cudaStream_t s = mp->ctx->stream;
+    if (mp->k.periodic)
+    {
+        if (mp->strategy == 0)
+            k_mp_first_periodic<D, true><<<grid_for(n, blk), blk, 0, s>>>(n, mp->k, mp->a, mp->f_offset, mp->in, step,
+                                                                         ac);
+        else
+            k_mp_first_periodic<D, false><<<grid_for(n, blk), blk, 0, s>>>(n, mp->k, mp->a, mp->f_offset, mp->in, step,
+                                                                          ac);
+    }
+    else if (ordered_lanes(mp) > 1)
+        k_mp_first_ordered<D, kOrderedLanes><<<grid_for(kOrderedLanes * n, blk), blk, 0, s>>>(n, mp->k, mp->a, mp->w,
+                                                                                             mp->in, mp->wl, step, ac);
+    else if (mp->strategy != 1)
+        mp->order_active ? launch_first<D, true, true>(mp, blk, step, ac) : launch_first<D, true, false>(mp, blk, step, ac);
+    else
+        mp->order_active ? launch_first<D, false, true>(mp, blk, step, ac)
+                         : launch_first<D, false, false>(mp, blk, step, ac);
+}
+
+template <int D, class Step>
+void sweep_second(sphx_mp mp, unsigned blk, const Step &step)
+{
+    const size_t n = mp->n;
+    cudaStream_t s = mp->ctx->stream;
+    if (mp->k.periodic)
+        mp->strategy == 0 ? launch_second_periodic<D, true>(mp, blk, step)
+                          : launch_second_periodic<D, false>(mp, blk, step);
+    else if (ordered_lanes(mp) > 1)
+        k_mp_second_ordered<D, kOrderedLanes><<<grid_for(kOrderedLanes * n, blk), blk, 0, s>>>(
+            n, mp->k, mp->a, mp->w, mp->in, mp->wl, step, mp->slots + 1);
+    else if (mp->strategy != 1)
+        mp->order_active ? launch_second<D, true, true>(mp, blk, step) : launch_second<D, true, false>(mp, blk, step);
+    else
+        mp->order_active ? launch_second<D, false, true>(mp, blk, step) : launch_second<D, false, false>(mp, blk, step);
+}
+
+// Whether the sub-steps of a step take their sizes from the device record: the strategies 0
+// and 1; a step that delivers host rows must know its last sub-step beforehand, and a
+// profiled one brackets every sweep with events.  Many particles: the sweeps look their step
+// up and test for the end, which costs them up to 5 % (3D, 3,340,000 particles: 2nd half 818
+// -> 866 us), while a round trip per sub-step is a small share of the step.
+bool planned(sphx_mp mp)
+{
+    const size_t few = mp->dim == 3 ? 250000 : 1000000;
+    return mp->n > 0 && mp->n < few && mp->strategy <= 1 && !mp->lists_tiled && mp->lists_strategy != 2 && !mp->host_pos &&
+           !mp->profiling;
+}
+
+// Enqueues sub-step s of a plan.
+template <int D>
+int planned_substep(sphx_mp mp, const StepPlan &plan, int s)
+{
+    sphx_ctx ctx = mp->ctx;
+    const size_t n = mp->n;
+    const unsigned blk = unsigned(mp->block);
+    k_mp_init1_planned<<<grid_for(n, 256 * kInitItems), 256, 0, ctx->stream>>>(n, mp->a.drho, mp->a.drho_dt, mp->a.dyn, mp->a.pres,
+                                                                  mp->k.p.p0_over_rho0, plan, s);
+    SPHX_LAUNCHED(ctx);
+    const StepArg step{plan.rec, plan.Dt, s};
+    sweep_first<D>(mp, blk, step, &plan.rec->ac[(s + 1) & 1]);
+    SPHX_LAUNCHED(ctx);
+    sweep_second<D>(mp, blk, step);
+    SPHX_LAUNCHED(ctx);
+    return SPHX_OK;
+}
+
+// The relaxation of one advection step by plan: as many sub-steps enqueued as the first step
+// size predicts, one look at the record, more where the prediction fell short.
+template <int D>
+int planned_relaxation(sphx_mp mp, int loop_style, double Dt, double ac, int *count)
+{
+    cudaStream_t s = mp->ctx->stream;
+    const double cfl_h = mp->k.acoustic_cfl * mp->k.p.h;
+    double dt = cfl_h / (ac + kTinyReal), relaxation = 0;
+    if (mp->k.periodic && loop_style == 0)
+        dt = std::min(dt, Dt);
+    StepPlan plan{reinterpret_cast<StepRecord *>(mp->slots + kSlots), mp->slots, Dt, cfl_h, 0.0, mp->acoustic_dt,
+                  loop_style, mp->k.periodic ? 1 : 0};
+    const StepRecord *rec = reinterpret_cast<const StepRecord *>(mp->h_slots + kSlots);
+    *count = 0;
+    while (relaxation < Dt)
+    {
+        const double left = std::ceil((Dt - relaxation) / dt);
+        const int batch = left >= 1.0 && left < double(kRecordSteps) ? int(left) : (left < 1.0 ? 1 : kRecordSteps);
+        plan.relax0 = relaxation;
+        for (int q = 0; q < batch; ++q)
+            SPHX_TRY(planned_substep<D>(mp, plan, q));
+        SPHX_CUDA(cudaMemcpyAsync(mp->h_slots, mp->slots, (kSlots + kRecordWords) * sizeof(unsigned long long),
+                                  cudaMemcpyDeviceToHost, s));
+        SPHX_CUDA(cudaStreamSynchronize(s));
+        int done = 0;
+        while (done < batch && rec->relax[done] < Dt)
+            ++done;
+        // the acoustic maximum of the last sub-step run, where the next step looks for it
+        const int last = done & 1;
+        SPHX_CUDA(cudaMemcpyAsync(mp->slots, &plan.rec->ac[last], sizeof(unsigned long long), cudaMemcpyDeviceToDevice,
+                                  s));
+        mp->h_slots[0] = rec->ac[last];
+        double next = cfl_h / (from_ordered_bits(mp->h_slots[0]) + kTinyReal);
+        for (int q = 0; q < done; ++q)
+        {
+            // loop style 1 takes the step size after the sub-step it follows
+            const double taken = loop_style == 0 ? rec->dt[q] : (q + 1 < batch ? rec->dt[q + 1] : next);
+            relaxation += taken;
+            mp->physical_time += taken;
+            mp->acoustic_dt = taken;
+        }
+        plan.first_dt = mp->acoustic_dt;
+        *count += done;
+        dt = next;
+    }
+    return SPHX_OK;
+}
+
 // One acoustic sub-step; deliver: the last of an advection step with host rows registered.
 template <int D>
 int substep(sphx_mp mp, double dt, bool deliver = false)
@@ -1512,6 +1778,7 @@ int substep(sphx_mp mp, double dt, bool deliver = false)
     if (!mp->k.periodic && (mp->strategy == 2) != (mp->lists_strategy == 2))
         SPHX_TRY(launch_build<D>(mp));
     unsigned blk = unsigned(mp->block);
+    mp->slots_read = false;
     k_mp_init1<<<grid_for(n, 256), 256, 0, s>>>(n, mp->a.drho, mp->a.drho_dt, mp->a.dyn, mp->a.pres,
                                                 mp->k.p.p0_over_rho0, float(0.5 * dt));
     SPHX_LAUNCHED(ctx);
@@ -1525,16 +1792,7 @@ int substep(sphx_mp mp, double dt, bool deliver = false)
         }
     if (e[0])
         SPHX_CUDA(cudaEventRecord(e[0], s));
-    if (mp->k.periodic)
-    {
-        if (mp->strategy == 0)
-            k_mp_first_periodic<D, true><<<grid_for(n, blk), blk, 0, s>>>(n, mp->k, mp->a, mp->f_offset, mp->in, dt,
-                                                                         mp->slots);
-        else
-            k_mp_first_periodic<D, false><<<grid_for(n, blk), blk, 0, s>>>(n, mp->k, mp->a, mp->f_offset, mp->in, dt,
-                                                                          mp->slots);
-    }
-    else if (mp->lists_tiled)
+    if (mp->lists_tiled)
         SPHX_TRY(launch_first_tiled<D>(mp, blk, dt));
     else if (mp->strategy == 3)
         SPHX_TRY(launch_first_async<D>(mp, blk, dt));
@@ -1542,10 +1800,8 @@ int substep(sphx_mp mp, double dt, bool deliver = false)
         SPHX_TRY(launch_first_persistent<D>(mp, blk, dt));
     else if (strategy_lanes(mp->strategy))
         launch_first_lanes<D>(mp, blk, dt);
-    else if (mp->strategy != 1)
-        mp->order_active ? launch_first<D, true, true>(mp, blk, dt) : launch_first<D, true, false>(mp, blk, dt);
     else
-        mp->order_active ? launch_first<D, false, true>(mp, blk, dt) : launch_first<D, false, false>(mp, blk, dt);
+        sweep_first<D>(mp, blk, dt, mp->slots);
     SPHX_LAUNCHED(ctx);
     if (deliver)
         SPHX_TRY(deliver_rows<D>(mp, kRowsVelocity));
@@ -1553,14 +1809,7 @@ int substep(sphx_mp mp, double dt, bool deliver = false)
         SPHX_CUDA(cudaEventRecord(e[1], s));
     if (e[2])
         SPHX_CUDA(cudaEventRecord(e[2], s));
-    if (mp->k.periodic)
-    {
-        if (mp->strategy == 0)
-            launch_second_periodic<D, true>(mp, blk, dt);
-        else
-            launch_second_periodic<D, false>(mp, blk, dt);
-    }
-    else if (mp->lists_tiled)
+    if (mp->lists_tiled)
         SPHX_TRY(launch_second_tiled<D>(mp, blk, dt));
     else if (mp->strategy == 3)
         SPHX_TRY(launch_second_async<D>(mp, blk, dt));
@@ -1568,10 +1817,8 @@ int substep(sphx_mp mp, double dt, bool deliver = false)
         SPHX_TRY(launch_second_persistent<D>(mp, blk, dt));
     else if (strategy_lanes(mp->strategy))
         launch_second_lanes<D>(mp, blk, dt);
-    else if (mp->strategy != 1)
-        mp->order_active ? launch_second<D, true, true>(mp, blk, dt) : launch_second<D, true, false>(mp, blk, dt);
     else
-        mp->order_active ? launch_second<D, false, true>(mp, blk, dt) : launch_second<D, false, false>(mp, blk, dt);
+        sweep_second<D>(mp, blk, dt);
     SPHX_LAUNCHED(ctx);
     if (deliver)
         SPHX_TRY(deliver_rows<D>(mp, kRowsPosition));
@@ -1584,8 +1831,14 @@ template <int D>
 int advection_step(sphx_mp mp, int loop_style, int *substeps, double *adv_dt)
 {
     SPHX_TRY(settle_configuration(mp));
-    double adv_max;
-    SPHX_TRY(read_slot(mp, 1, &adv_max));
+    if (!mp->slots_read)
+    {
+        SPHX_CUDA(cudaMemcpyAsync(mp->h_slots, mp->slots, 2 * sizeof(unsigned long long), cudaMemcpyDeviceToHost,
+                                  mp->ctx->stream));
+        SPHX_CUDA(cudaStreamSynchronize(mp->ctx->stream));
+    }
+    mp->slots_read = false;
+    const double adv_max = from_ordered_bits(mp->h_slots[1]);
     double Dt = mp->k.advection_cfl * mp->k.p.h / (std::max(std::sqrt(adv_max), mp->k.U_ref) + kTinyReal);
     if (mp->n > 0)
     {
@@ -1598,6 +1851,12 @@ int advection_step(sphx_mp mp, int loop_style, int *substeps, double *adv_dt)
     double relaxation = 0, dt = mp->acoustic_dt;
     int count = 0;
     bool delivered = false;
+    if (planned(mp))
+    {
+        SPHX_TRY(planned_relaxation<D>(mp, loop_style, Dt, from_ordered_bits(mp->h_slots[0]), &count));
+        dt = mp->acoustic_dt;
+        relaxation = Dt;
+    }
     while (relaxation < Dt)
     {
         double ac;
@@ -1817,7 +2076,7 @@ extern "C" int sphx_mp_create(sphx_relation inner, sphx_relation wall, const sph
     mp->w.nw = nw;
     mp->in.count = mp->alloc<uint32_t>(n);
     mp->wl.count = mp->alloc<uint32_t>(n);
-    mp->slots = mp->alloc<unsigned long long>(12);
+    mp->slots = mp->alloc<unsigned long long>(kSlots + kRecordWords);
     mp->order = mp->alloc<uint32_t>(n);
     mp->tile_offset = mp->alloc<uint32_t>(nc + 1);
     mp->tiles = mp->alloc<uint32_t>(nc);
@@ -1829,7 +2088,7 @@ extern "C" int sphx_mp_create(sphx_relation inner, sphx_relation wall, const sph
         return bail(fail(SPHX_ERR_OUT_OF_MEMORY, "mixed-precision allocation failed"));
     if (cudaMemsetAsync(mp->slots, 0, 12 * sizeof(unsigned long long), ctx->stream) != cudaSuccess)
         return bail(fail(SPHX_ERR_CUDA, "slot initialisation failed"));
-    if (cudaMallocHost(&mp->h_slots, 12 * sizeof(unsigned long long)) != cudaSuccess)
+    if (cudaMallocHost(&mp->h_slots, (kSlots + kRecordWords) * sizeof(unsigned long long)) != cudaSuccess)
         return bail(fail(SPHX_ERR_OUT_OF_MEMORY, "pinned allocation failed"));
     if ((st = alloc_lists(mp, mp->in, D == 2 ? 24 : 96)) != SPHX_OK ||
         (st = alloc_lists(mp, mp->wl, D == 2 ? 16 : 64)) != SPHX_OK)
@@ -1974,13 +2233,13 @@ extern "C" int sphx_mp_create_periodic(sphx_body fb, const sphx_fluid_params *p,
     mp->noff = mp->alloc<float>(6 * n);
     mp->in.count = mp->alloc<uint32_t>(n);
     mp->wl.count = mp->alloc<uint32_t>(n);
-    mp->slots = mp->alloc<unsigned long long>(12);
+    mp->slots = mp->alloc<unsigned long long>(kSlots + kRecordWords);
     if (!mp->f_offset || !mp->w_offset || !mp->count || !mp->key || !mp->rank || !mp->perm || !mp->ncell ||
         !mp->noff || !mp->in.count || !mp->wl.count || !mp->slots)
         return bail(fail(SPHX_ERR_OUT_OF_MEMORY, "mixed-precision allocation failed"));
     if (cudaMemsetAsync(mp->slots, 0, 12 * sizeof(unsigned long long), ctx->stream) != cudaSuccess)
         return bail(fail(SPHX_ERR_CUDA, "slot initialisation failed"));
-    if (cudaMallocHost(&mp->h_slots, 12 * sizeof(unsigned long long)) != cudaSuccess)
+    if (cudaMallocHost(&mp->h_slots, (kSlots + kRecordWords) * sizeof(unsigned long long)) != cudaSuccess)
         return bail(fail(SPHX_ERR_OUT_OF_MEMORY, "pinned allocation failed"));
     if ((st = alloc_lists(mp, mp->in, D == 2 ? 24 : 96)) != SPHX_OK || (st = alloc_lists(mp, mp->wl, 1)) != SPHX_OK)
         return bail(st);

@@ -337,6 +337,14 @@ struct Kahan
         c = (t - s) - y;
         s = t;
     }
+    // adds a b, rounded once with the correction
+    __device__ __forceinline__ void add_product(float a, float b)
+    {
+        float y = fmaf(a, b, -c);
+        float t = s + y;
+        c = (t - s) - y;
+        s = t;
+    }
     __device__ __forceinline__ float value() const { return s - c; }
 };
 
@@ -403,6 +411,19 @@ struct Acc
         k.add(part);
         part = 0.f;
     }
+    // Adds the partials of the first m lanes of this lane's group of L, in lane order.
+    template <int L>
+    __device__ __forceinline__ void merge(unsigned mask, unsigned m)
+    {
+#pragma unroll
+        for (int q = 0; q < L; ++q)
+        {
+            const float x = __shfl_sync(mask, part, q, L);
+            if (unsigned(q) < m)
+                k.add(x);
+        }
+        part = 0.f;
+    }
     __device__ __forceinline__ float value() const { return k.value(); }
 };
 
@@ -419,6 +440,19 @@ struct Acc2
         const float2 t = f2_add(s, y);
         c = f2_sub(f2_sub(t, s), y);
         s = t;
+        part = make_float2(0.f, 0.f);
+    }
+    template <int L>
+    __device__ __forceinline__ void merge(unsigned mask, unsigned m) // as Acc::merge
+    {
+        const float2 own = part;
+#pragma unroll
+        for (int q = 0; q < L; ++q)
+        {
+            part = make_float2(__shfl_sync(mask, own.x, q, L), __shfl_sync(mask, own.y, q, L));
+            if (unsigned(q) < m)
+                flush();
+        }
         part = make_float2(0.f, 0.f);
     }
     __device__ __forceinline__ float x() const { return s.x - c.x; }
@@ -530,14 +564,15 @@ __device__ __forceinline__ float dot(const float *a, const float *b)
 // 1 / r (0 for coincident particles, whose kernel gradient is zero).
 __device__ __forceinline__ float inv_dist(float r2) { return r2 > 0.f ? rsqrtf(r2) : 0.f; }
 
-// Wendland C2 W(r) = fW t^4 (1 + 2q), t = 1 - q/2.
-__device__ __forceinline__ float wc2_W(float fW, float inv_h, float r)
+// Wendland C2 W(r) / fW = t^4 (1 + 2q), t = 1 - q/2.
+__device__ __forceinline__ float wc2_shape(float inv_h, float r)
 {
     float q = r * inv_h;
     float t = 1.0f - 0.5f * q;
     float t2 = t * t;
-    return fW * (t2 * t2 * (1.0f + 2.0f * q));
+    return t2 * t2 * (1.0f + 2.0f * q);
 }
+__device__ __forceinline__ float wc2_W(float fW, float inv_h, float r) { return fW * wc2_shape(inv_h, r); }
 // dW(r) V = c (q - 2)^3 q with c = fdW 5/8 V.
 __device__ __forceinline__ float wc2_dWV(float c, float inv_h, float r)
 {
@@ -709,6 +744,14 @@ __device__ __forceinline__ unsigned lane_in_group()
     return LANES == 1 ? 0u : (threadIdx.x & unsigned(LANES - 1));
 }
 
+// The lanes of this lane's group of LANES, as a warp mask.
+template <int LANES>
+__device__ __forceinline__ unsigned group_lanes()
+{
+    const unsigned lane = threadIdx.x & 31u;
+    return ((1u << LANES) - 1u) << (lane & ~unsigned(LANES - 1));
+}
+
 // Sum of v over the LANES lanes of this lane's group (consecutive lanes, LANES a power of
 // two dividing 32); every lane of the group gets the sum.
 template <int LANES>
@@ -796,6 +839,57 @@ __device__ __forceinline__ void list_sweep(size_t i, size_t n, const MPNeighbors
             pair(load(j));
     }
     flush();
+}
+
+// list_sweep shared by L consecutive lanes with the sums of one lane, bit for bit: each
+// lane takes whole groups of kGroup neighbours (a plain partial sum each), and merge(m) adds
+// the m partials of a round to the compensated sums in list order; every lane ends with the
+// sums.  For few particles: a thread's chain of dependent gathers is L times shorter, and L
+// times as many warps hide it (3D dam break, 26,720 particles: 1st / 2nd half 33.7 / 48.1 us
+// with one lane).
+template <int U, int L, class Load, class Pair, class Merge>
+__device__ __forceinline__ void list_sweep_ordered(size_t i, size_t n, const MPNeighbors &l, Load &&load, Pair &&pair,
+                                                   Merge &&merge)
+{
+    static_assert(kGroup % U == 0, "groups hold whole unrolled batches");
+    const unsigned c = min(l.count[i], l.cap), sub = lane_in_group<L>();
+    const unsigned groups = c / kGroup + 1; // the last one holds the remainder
+    const uint32_t *J = l.J + i;
+    for (unsigned g = 0; g < groups; g += L)
+    {
+        const unsigned s0 = (g + sub) * kGroup;
+        if (s0 + kGroup <= c)
+        {
+            uint32_t jj[kGroup];
+#pragma unroll
+            for (int u = 0; u < kGroup; ++u)
+                jj[u] = __ldg(&J[size_t(s0 + u) * n]);
+#pragma unroll
+            for (int h = 0; h < kGroup; h += U)
+            {
+                decltype(load(0u)) rec[U];
+                bool ok[U];
+#pragma unroll
+                for (int u = 0; u < U; ++u)
+                {
+                    ok[u] = entry_ok(jj[h + u], l);
+                    rec[u] = ok[u] ? load(jj[h + u]) : decltype(load(0u)){};
+                }
+#pragma unroll
+                for (int u = 0; u < U; ++u)
+                    if (ok[u])
+                        pair(rec[u]);
+            }
+        }
+        else
+            for (unsigned s = s0; s < c; ++s)
+            {
+                const uint32_t j = __ldg(&J[size_t(s) * n]);
+                if (entry_ok(j, l))
+                    pair(load(j));
+            }
+        merge(min(unsigned(L), groups - g));
+    }
 }
 
 // ---------------------------------------------------------------- asynchronous gathers
@@ -907,6 +1001,10 @@ __device__ __forceinline__ void cell_sweep(const Visit &v, const uint32_t *offse
     flush();
 }
 
+// The step size of a sweep, given by value or (mixed.cu) looked up when the sums are done, so
+// that it takes no registers during them.
+__device__ __forceinline__ double step_size(double dt) { return dt; }
+
 struct FirstRec
 {
     float4 g;
@@ -924,9 +1022,10 @@ struct SecondRec
 // that depth (ring: slots for geo0 in a, the pressure in c).
 // LANES > 1: the stored lists, LANES consecutive lanes on particle i (list slots strided
 // over the lanes, sums combined by shuffles); the first lane of the group writes the state
-// and returns the candidate, the others return -1e300.
-template <int D, bool LISTS, int DEPTH = 0, int LANES = 1>
-__device__ __forceinline__ double first_particle(size_t i, size_t n, const MPParams &k, const Visit &v, double dt,
+// and returns the candidate, the others return -1e300.  ORDERED: the lanes share the list
+// as list_sweep_ordered does, with the results of one lane.
+template <int D, bool LISTS, int DEPTH = 0, int LANES = 1, bool ORDERED = false, class Step = double>
+__device__ __forceinline__ double first_particle(size_t i, size_t n, const MPParams &k, const Visit &v, const Step &step,
                                                  const MPState &f, const MPWallData &w, const MPNeighbors &in,
                                                  const MPNeighbors &wl, const AsyncRing<DEPTH> *ring = nullptr)
 {
@@ -974,6 +1073,16 @@ __device__ __forceinline__ double first_particle(size_t i, size_t n, const MPPar
         auto read = [&](unsigned slot) { return FirstRec{rg.a[rg.at(slot)], rg.c[rg.at(slot)]}; };
         list_sweep_async<DEPTH>(i, n, in, rg, issue, read, pair, flush);
     }
+    else if constexpr (ORDERED)
+    {
+        const unsigned mask = group_lanes<LANES>();
+        list_sweep_ordered<kUnrollFirst, LANES>(i, n, in, load, pair, [&](unsigned m) {
+            force01.template merge<LANES>(mask, m);
+            if (D == 3)
+                force2.template merge<LANES>(mask, m);
+            rdis.template merge<LANES>(mask, m);
+        });
+    }
     else if (LISTS)
         list_sweep<true, kUnrollFirst, LANES>(i, n, in, load, pair, flush, lane_in_group<LANES>());
     else
@@ -1002,12 +1111,23 @@ __device__ __forceinline__ double first_particle(size_t i, size_t n, const MPPar
         wrdis.flush();
     };
     auto wload = [&](uint32_t j) { return __ldg(&w.geo[j]); };
-    if (LISTS || DEPTH > 0)
+    if constexpr (ORDERED)
+    {
+        const unsigned mask = group_lanes<LANES>();
+        list_sweep_ordered<kUnrollFirst, LANES>(i, n, wl, wload, wpair, [&](unsigned m) {
+            wforce01.template merge<LANES>(mask, m);
+            if (D == 3)
+                wforce2.template merge<LANES>(mask, m);
+            wrdis.template merge<LANES>(mask, m);
+        });
+    }
+    else if (LISTS || DEPTH > 0)
         list_sweep<true, kUnrollFirst, LANES>(i, n, wl, wload, wpair, wflush, lane_in_group<LANES>());
     else
         cell_sweep<D, false>(v, v.w_offset, ci, k.gs_f, pib, oi, k.rc_sqr, k.rc_reach, ~size_t(0), w.geo, wload,
                              wpair, wflush);
 
+    constexpr int SUMS = ORDERED ? 1 : LANES; // ordered: every lane holds the sums
     const float fv[3] = {force01.x(), force01.y(), force2.value()};
     const float wv[3] = {wforce01.x(), wforce01.y(), wforce2.value()};
     const float rv = rdis.value();
@@ -1015,12 +1135,13 @@ __device__ __forceinline__ double first_particle(size_t i, size_t n, const MPPar
 #pragma unroll
     for (int d = 0; d < D; ++d)
     {
-        fsum[d] = group_sum<LANES>(fv[d]);
-        wfsum[d] = group_sum<LANES>(wv[d]);
+        fsum[d] = group_sum<SUMS>(fv[d]);
+        wfsum[d] = group_sum<SUMS>(wv[d]);
     }
-    const float rsum = group_sum<LANES>(rv), wrsum = group_sum<LANES>(wrdis.value());
+    const float rsum = group_sum<SUMS>(rv), wrsum = group_sum<SUMS>(wrdis.value());
     if (lane_in_group<LANES>() != 0)
         return -1.0e300;
+    const double dt = step_size(step);
     f.drho_dt[i] = (rsum * k.inv_z) * rho_i + (wrsum * k.inv_z) * rho_i;
     float v2 = 0.f;
     float vn[3] = {di.x, di.y, di.z};
@@ -1046,8 +1167,8 @@ __device__ __forceinline__ double first_particle(size_t i, size_t n, const MPPar
 // advection-time-step candidate max(|v|^2, 4 h |F + F_prior| / m).
 // DEPTH > 0: the stored lists with the neighbour records gathered through an AsyncRing of
 // that depth (ring: slots for geo0 in a, dyn in b).  LANES as first_particle.
-template <int D, bool LISTS, int DEPTH = 0, int LANES = 1>
-__device__ __forceinline__ double second_particle(size_t i, size_t n, const MPParams &k, const Visit &v, double dt,
+template <int D, bool LISTS, int DEPTH = 0, int LANES = 1, bool ORDERED = false, class Step = double>
+__device__ __forceinline__ double second_particle(size_t i, size_t n, const MPParams &k, const Visit &v, const Step &step,
                                                   const MPState &f, const MPWallData &w, const MPNeighbors &in,
                                                   const MPNeighbors &wl, const AsyncRing<DEPTH> *ring = nullptr)
 {
@@ -1134,6 +1255,18 @@ __device__ __forceinline__ double second_particle(size_t i, size_t n, const MPPa
         auto read = [&](unsigned slot) { return SecondRec{rg.a[rg.at(slot)], rg.b[rg.at(slot)]}; };
         list_sweep_async<DEPTH>(i, n, in, rg, issue, read, pair, flush);
     }
+    else if constexpr (ORDERED)
+    {
+        static_assert(SPHX_PACKED_SECOND, "the ordered form merges the packed sums");
+        const unsigned mask = group_lanes<LANES>();
+        list_sweep_ordered<kUnrollSecond, LANES>(i, n, in, load, pair, [&](unsigned m) {
+            pdis01.template merge<LANES>(mask, m);
+            if (D == 3)
+                zr.template merge<LANES>(mask, m);
+            else
+                rate.template merge<LANES>(mask, m);
+        });
+    }
     else if (LISTS)
         list_sweep<kPrefetchSecond, kUnrollSecond, LANES>(i, n, in, load, pair, flush, lane_in_group<LANES>());
     else
@@ -1164,12 +1297,23 @@ __device__ __forceinline__ double second_particle(size_t i, size_t n, const MPPa
             wdis2.flush();
     };
     auto wload = [&](uint32_t j) { return SecondRec{__ldg(&w.geo[j]), __ldg(&w.n[j])}; };
-    if (LISTS || DEPTH > 0)
+    if constexpr (ORDERED)
+    {
+        const unsigned mask = group_lanes<LANES>();
+        list_sweep_ordered<kUnrollSecond, LANES>(i, n, wl, wload, wpair, [&](unsigned m) {
+            wrate.template merge<LANES>(mask, m);
+            wdis01.template merge<LANES>(mask, m);
+            if (D == 3)
+                wdis2.template merge<LANES>(mask, m);
+        });
+    }
+    else if (LISTS || DEPTH > 0)
         list_sweep<false, kUnrollSecond, LANES>(i, n, wl, wload, wpair, wflush, lane_in_group<LANES>());
     else
         cell_sweep<D, false>(v, v.w_offset, ci, k.gs_f, pib, oi, k.rc_sqr, k.rc_reach, ~size_t(0), w.geo, wload,
                              wpair, wflush);
 
+    constexpr int SUMS = ORDERED ? 1 : LANES;
     const bool zr_rate = SPHX_PACKED_SECOND && D == 3;
     const float pv[3] = {SPHX_PACKED_SECOND ? pdis01.x() : pdis[0].value(),
                          SPHX_PACKED_SECOND ? pdis01.y() : pdis[1].value(),
@@ -1180,12 +1324,13 @@ __device__ __forceinline__ double second_particle(size_t i, size_t n, const MPPa
 #pragma unroll
     for (int d = 0; d < D; ++d)
     {
-        psum[d] = group_sum<LANES>(pv[d]);
-        wpsum[d] = group_sum<LANES>(wv[d]);
+        psum[d] = group_sum<SUMS>(pv[d]);
+        wpsum[d] = group_sum<SUMS>(wv[d]);
     }
-    const float ratesum = group_sum<LANES>(rate_v), wratesum = group_sum<LANES>(wrate.value());
+    const float ratesum = group_sum<SUMS>(rate_v), wratesum = group_sum<SUMS>(wrate.value());
     if (lane_in_group<LANES>() != 0)
         return -1.0e300;
+    const double dt = step_size(step);
     float drho_dt = f.drho_dt[i] + ratesum * rho_i + wratesum * rho_i;
     f.drho_dt[i] = drho_dt;
     f.drho[i] = f.drho[i] + drho_dt * float(0.5 * dt);
@@ -1235,7 +1380,7 @@ __device__ __forceinline__ void build_particle(size_t i, size_t n, const MPParam
                                             if (cnt < in.cap)
                                                 in.J[size_t(cnt) * n + i] = j;
                                             ++cnt;
-                                            sigma.add(wc2_W(k.fW, k.inv_h, sqrtf(r2)));
+                                            sigma.add_product(k.fW, wc2_shape(k.inv_h, sqrtf(r2)));
                                         }
                                     });
     Kahan wsig;
@@ -1253,7 +1398,7 @@ __device__ __forceinline__ void build_particle(size_t i, size_t n, const MPParam
                                              if (wc < wl.cap)
                                                  wl.J[size_t(wc) * n + i] = j;
                                              ++wc;
-                                             wsig.add(wc2_W(k.fW, k.inv_h, sqrtf(r2)));
+                                             wsig.add_product(k.fW, wc2_shape(k.inv_h, sqrtf(r2)));
                                          }
                                      });
     in.count[i] = cnt;
@@ -1261,6 +1406,81 @@ __device__ __forceinline__ void build_particle(size_t i, size_t n, const MPParam
     warp_atomic_max(&max_counts[0], cnt);
     warp_atomic_max(&max_counts[1], wc);
     // rho_sum - rho0 = rho0 (W0 + sum W - sigma0) / sigma0 + wall term
+    double dsig = (double(sigma.s) - k.sigma0) - double(sigma.c) + double(k.fW);
+    f.drho_sum[i] = float(dsig) * k.rho0_over_sigma0 + wsig.value() * k.wall_factor;
+}
+
+// Tests the candidates [b, e) of a run side by side in the L lanes of a group:
+// test(j, r2) -> accepted; accepted candidates take the next list slots in candidate order,
+// and their kernel values enter the sum one by one in that order, in every lane.
+template <int L, class Test>
+__device__ __forceinline__ void run_in_lanes(uint32_t b, uint32_t e, size_t i, size_t n, const MPParams &k,
+                                             const MPNeighbors &l, uint32_t tag, unsigned &cnt, Kahan *sum, Test &&test)
+{
+    const unsigned mask = group_lanes<L>(), sub = lane_in_group<L>(), first = (threadIdx.x & 31u) & ~unsigned(L - 1);
+    for (uint32_t j0 = b; j0 < e; j0 += L)
+    {
+        const uint32_t j = j0 + sub;
+        float r2 = 0.0f;
+        const bool take = j < e && test(j, r2);
+        const unsigned votes = (__ballot_sync(mask, take) & mask) >> first;
+        const unsigned slot = cnt + __popc(votes & ((1u << sub) - 1u));
+        if (take && slot < l.cap)
+            l.J[size_t(slot) * n + i] = j | tag;
+        cnt += __popc(votes);
+        if (sum)
+        {
+            const float w = take ? wc2_shape(k.inv_h, sqrtf(r2)) : 0.0f;
+#pragma unroll
+            for (int q = 0; q < L; ++q)
+            {
+                const float x = __shfl_sync(mask, w, q, L);
+                if ((votes >> q) & 1u)
+                    sum->add_product(k.fW, x);
+            }
+        }
+    }
+}
+
+// build_particle shared by L lanes, with its lists and sums bit for bit.
+template <int D, int L>
+__device__ __forceinline__ void build_particle_lanes(size_t i, size_t n, const MPParams &k, const Visit &v,
+                                                     const MPState &f, const MPWallData &w, const MPNeighbors &in,
+                                                     const MPNeighbors &wl, unsigned int *max_counts)
+{
+    const float4 gi = f.geo0[i];
+    int ci[3] = {0, 0, 0};
+    unpack_cell<D>(__float_as_uint(gi.w), ci);
+    const float oi[3] = {gi.x, gi.y, gi.z};
+    Kahan sigma, wsig;
+    unsigned cnt = 0, wc = 0;
+    const RunDx<D> rd(k.gs_f, ci, oi);
+    for_each_candidate_run<D, true>(v.m, v.cell_base, v.f_offset, ci, Reach(oi, k.gs_f, k.rc_reach),
+                                    [&](int x, int y, uint32_t b, uint32_t e) {
+                                        const float dcx = rd.column(x), dcy = rd.column_y(y);
+                                        run_in_lanes<L>(b, e, i, n, k, in, 0u, cnt, &sigma, [&](uint32_t j, float &r2) {
+                                            float dx[3];
+                                            rd.dx(dcx, dcy, f.geo0[j], dx);
+                                            r2 = sq<D>(dx);
+                                            return j != uint32_t(i) && r2 < k.rc_sqr;
+                                        });
+                                    });
+    for_each_candidate_run<D, false>(v.m, v.cell_base, v.w_offset, ci, Reach(oi, k.gs_f, k.rc_reach),
+                                     [&](int x, int y, uint32_t b, uint32_t e) {
+                                         const float dcx = rd.column(x), dcy = rd.column_y(y);
+                                         run_in_lanes<L>(b, e, i, n, k, wl, 0u, wc, &wsig, [&](uint32_t j, float &r2) {
+                                             float dx[3];
+                                             rd.dx(dcx, dcy, w.geo[j], dx);
+                                             r2 = sq<D>(dx);
+                                             return r2 < k.rc_sqr;
+                                         });
+                                     });
+    warp_atomic_max(&max_counts[0], cnt);
+    warp_atomic_max(&max_counts[1], wc);
+    if (lane_in_group<L>() != 0)
+        return;
+    in.count[i] = cnt;
+    wl.count[i] = wc;
     double dsig = (double(sigma.s) - k.sigma0) - double(sigma.c) + double(k.fW);
     f.drho_sum[i] = float(dsig) * k.rho0_over_sigma0 + wsig.value() * k.wall_factor;
 }
@@ -1403,9 +1623,9 @@ struct SecondRecP
 // 1st half of one particle of a periodic flow without walls (Integration1stHalfInnerRiemann):
 // pressure force, density-rate dissipation, v += (F_prior + F) / m dt, first position
 // half-step.  Returns c0 + |v|.
-template <int D, bool LISTS>
+template <int D, bool LISTS, class Step = double>
 __device__ __forceinline__ double first_particle_periodic(size_t i, size_t n, const MPParams &k, const MeshDev &m,
-                                                          const uint32_t *f_offset, double dt, const MPState &f,
+                                                          const uint32_t *f_offset, const Step &step, const MPState &f,
                                                           const MPNeighbors &in)
 {
     const float4 gi = f.geo0[i];
@@ -1448,6 +1668,7 @@ __device__ __forceinline__ double first_particle_periodic(size_t i, size_t n, co
     else
         cell_sweep_periodic<D>(m, f_offset, ci, k, pib, oi, i, f.geo0, load, pair, flush);
 
+    const double dt = step_size(step);
     f.drho_dt[i] = (rdis.value() * k.inv_z) * rho_i;
     float v2 = 0.f;
     float vn[3] = {di.x, di.y, di.z};
@@ -1470,9 +1691,9 @@ __device__ __forceinline__ double first_particle_periodic(size_t i, size_t n, co
 // 2nd half of one particle of a periodic flow: Integration2ndHalfInnerRiemann (RIEMANN),
 // or Integration2ndHalfInnerNoRiemann, whose pressure dissipation is zero, so the force
 // sum is left out.  Returns max(|v|^2, 4 h |F + F_prior| / m).
-template <int D, bool LISTS, bool RIEMANN>
+template <int D, bool LISTS, bool RIEMANN, class Step = double>
 __device__ __forceinline__ double second_particle_periodic(size_t i, size_t n, const MPParams &k, const MeshDev &m,
-                                                           const uint32_t *f_offset, double dt, const MPState &f,
+                                                           const uint32_t *f_offset, const Step &step, const MPState &f,
                                                            const MPNeighbors &in)
 {
     const float4 gi = f.geo0[i];
@@ -1535,6 +1756,7 @@ __device__ __forceinline__ double second_particle_periodic(size_t i, size_t n, c
     else
         cell_sweep_periodic<D>(m, f_offset, ci, k, pib, oi, i, f.geo0, load, pair, flush);
 
+    const double dt = step_size(step);
     float drho_dt = f.drho_dt[i] + rate.value() * rho_i;
     f.drho_dt[i] = drho_dt;
     f.drho[i] = f.drho[i] + drho_dt * float(0.5 * dt);
