@@ -148,7 +148,6 @@ __global__ void k_b_sort_segments(size_t nseg, const uint32_t *__restrict__ offs
         sort_segment(idx, offset[c], offset[c + 1]);
 }
 
-__global__ void k_b_set_total(uint32_t *offset, size_t ncells, uint32_t total) { offset[ncells] = total; }
 
 template <int D>
 __global__ void k_b_gather(size_t n, const uint32_t *__restrict__ perm, const uint32_t *__restrict__ ncell,
@@ -513,8 +512,7 @@ int b_alloc_lists(sphx_batch bt, MPNeighbors &l, unsigned cap)
 // Offsets and cell-ordered permutation of n hashed particles (key/rank/cnt filled).
 int b_enqueue_sort(sphx_batch bt, cudaStream_t s, size_t n, uint32_t *offset)
 {
-    SPHX_TRY(exclusive_scan_into(s, bt->cnt, offset, bt->ncells, bt->scan_tiles));
-    k_b_set_total<<<1, 1, 0, s>>>(offset, bt->ncells, uint32_t(n));
+    SPHX_TRY(exclusive_scan_into(s, bt->cnt, offset, bt->ncells, bt->scan_tiles, offset + bt->ncells));
     SPHX_CUDA(cudaGetLastError());
     if (n == 0)
         return SPHX_OK;

@@ -109,9 +109,12 @@ __global__ void k_scan_tile_prefix(uint32_t *__restrict__ tile_sums, size_t ntil
         *total_out = carry;
 }
 
-// Pass 3: scan inside each tile, offset by the tile prefix.
+// Last pass: scan inside each tile.  PREFIXED: tiles holds the tiles' prefixes; else it holds
+// their sums, and every block adds up those before its own (few tiles: one launch less).
+// *total_out, when given, gets the sum of everything.
+template <bool PREFIXED>
 __global__ void k_scan_apply(const uint32_t *__restrict__ in, uint32_t *__restrict__ out, size_t n,
-                             const uint32_t *__restrict__ tile_prefix)
+                             const uint32_t *__restrict__ tiles, uint32_t *__restrict__ total_out)
 {
     __shared__ uint32_t sw[32];
     size_t base = size_t(blockIdx.x) * kScanTile + size_t(threadIdx.x) * kScanItems;
@@ -123,8 +126,20 @@ __global__ void k_scan_apply(const uint32_t *__restrict__ in, uint32_t *__restri
         v[k] = base + k < n ? in[base + k] : 0u;
         s += v[k];
     }
+    uint32_t before = 0;
+    if (PREFIXED)
+        before = tiles[blockIdx.x];
+    else
+    {
+        uint32_t mine = 0;
+        for (unsigned t = threadIdx.x; t < blockIdx.x; t += blockDim.x)
+            mine += tiles[t];
+        block_exclusive_scan(mine, sw, before);
+    }
     uint32_t total;
-    uint32_t run = tile_prefix[blockIdx.x] + block_exclusive_scan(s, sw, total);
+    uint32_t run = before + block_exclusive_scan(s, sw, total);
+    if (total_out && blockIdx.x == gridDim.x - 1 && threadIdx.x == 0)
+        *total_out = before + total;
 #pragma unroll
     for (unsigned k = 0; k < kScanItems; ++k)
         if (base + k < n)
@@ -141,9 +156,6 @@ __global__ void k_count_keys(size_t n, const uint32_t *__restrict__ key, uint32_
     if (i < n)
         rank[i] = atomicAdd(&count[key[i]], 1u);
 }
-
-// offset[nkeys] = total, closing the CellOffset array (cell_linked_list.cpp:171-174).
-__global__ void k_set_total(uint32_t *offset, uint32_t nkeys, uint32_t total) { offset[nkeys] = total; }
 
 __global__ void k_scatter(size_t n, const uint32_t *__restrict__ cell_of, const uint32_t *__restrict__ rank,
                           const uint32_t *__restrict__ offset, uint32_t *__restrict__ particle_index)
@@ -198,28 +210,30 @@ __global__ void k_entry_init(size_t n, int dim, const double *__restrict__ pos, 
     eidx[i] = uint32_t(i);
 }
 
-// 1 for the entries that get an image on this side: lower < x < lower + rc (side 0) or
-// upper - rc < x < upper (side 1), strict as in domain_bounding.cpp:20-50
-__global__ void k_image_flags(size_t n_cur, size_t E, const double *__restrict__ epos, int axis, double lo, double hi,
-                              uint32_t *__restrict__ flag)
+// The entries that get an image on each side of an axis: flag[e] for lower < x < lower + rc,
+// flag[n_cur + e] for upper - rc < x < upper, strict as in domain_bounding.cpp:20-50.
+__global__ void k_image_flags(size_t n_cur, size_t E, const double *__restrict__ epos, int axis, double lo, double up,
+                              double rc, uint32_t *__restrict__ flag)
 {
     size_t e = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
     if (e >= n_cur)
         return;
     double x = epos[axis * E + e];
-    flag[e] = (x > lo && x < hi) ? 1u : 0u;
+    flag[e] = (x > lo && x < lo + rc) ? 1u : 0u;
+    flag[n_cur + e] = (x > up - rc && x < up) ? 1u : 0u;
 }
 
+// The images of both sides after the current entries: those of the lower side, then those of
+// the upper one, in entry order (the scan runs over the flags of both).
 __global__ void k_image_emit(size_t n_cur, int dim, size_t E, double *__restrict__ epos, uint32_t *__restrict__ eidx,
-                             const uint32_t *__restrict__ flag, const uint32_t *__restrict__ scan, size_t base,
-                             int axis, double shift)
+                             const uint32_t *__restrict__ flag, const uint32_t *__restrict__ scan, int axis, double L)
 {
-    size_t e = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (e >= n_cur || !flag[e])
+    const size_t q = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
+    if (q >= 2 * n_cur || !flag[q])
         return;
-    size_t k = base + scan[e];
+    const size_t e = q < n_cur ? q : q - n_cur, k = n_cur + scan[q];
     for (int a = 0; a < dim; ++a)
-        epos[a * E + k] = epos[a * E + e] + (a == axis ? shift : 0.0);
+        epos[a * E + k] = epos[a * E + e] + (a == axis ? (q < n_cur ? L : -L) : 0.0);
     eidx[k] = eidx[e];
 }
 
@@ -339,39 +353,54 @@ __global__ void k_morton_rank_key(size_t n, const double *__restrict__ pos, Mesh
 
 namespace sphx
 {
-int exclusive_scan(sphx_ctx ctx, const uint32_t *d_in, uint32_t *d_out, size_t n)
+// Tiles up to which a block of the last pass adds up the tile sums before its own: 8 loads a
+// thread at most.
+constexpr size_t kDirectTiles = 8 * kBlock;
+
+static int scan_passes(cudaStream_t s, const uint32_t *d_in, uint32_t *d_out, size_t n, uint32_t *tiles, uint32_t *total_out,
+                int *launches)
+{
+    const size_t ntiles = (n + kScanTile - 1) / kScanTile;
+    *launches = 1;
+    if (ntiles > 1)
+    {
+        k_scan_tile_sums<<<unsigned(ntiles), kBlock, 0, s>>>(d_in, n, tiles);
+        SPHX_CUDA(cudaGetLastError());
+        ++*launches;
+    }
+    if (ntiles <= kDirectTiles)
+        k_scan_apply<false><<<unsigned(ntiles), kBlock, 0, s>>>(d_in, d_out, n, tiles, total_out);
+    else
+    {
+        k_scan_tile_prefix<<<1, 1024, 0, s>>>(tiles, ntiles, tiles + ntiles);
+        SPHX_CUDA(cudaGetLastError());
+        k_scan_apply<true><<<unsigned(ntiles), kBlock, 0, s>>>(d_in, d_out, n, tiles, total_out);
+        ++*launches;
+    }
+    SPHX_CUDA(cudaGetLastError());
+    return SPHX_OK;
+}
+
+int exclusive_scan(sphx_ctx ctx, const uint32_t *d_in, uint32_t *d_out, size_t n, uint32_t *total_out)
 {
     if (n == 0)
         return SPHX_OK;
-    size_t ntiles = (n + kScanTile - 1) / kScanTile;
-    SPHX_TRY(ctx->ensure_scratch((ntiles + 1) * sizeof(uint32_t)));
-    uint32_t *tiles = static_cast<uint32_t *>(ctx->d_scratch);
-    k_scan_tile_sums<<<unsigned(ntiles), kBlock, 0, ctx->stream>>>(d_in, n, tiles);
-    SPHX_LAUNCHED(ctx);
-    k_scan_tile_prefix<<<1, 1024, 0, ctx->stream>>>(tiles, ntiles, tiles + ntiles);
-    SPHX_LAUNCHED(ctx);
-    k_scan_apply<<<unsigned(ntiles), kBlock, 0, ctx->stream>>>(d_in, d_out, n, tiles);
-    SPHX_LAUNCHED(ctx);
+    SPHX_TRY(ctx->ensure_scratch(scan_scratch_entries(n) * sizeof(uint32_t)));
+    int launches = 0;
+    SPHX_TRY(scan_passes(ctx->stream, d_in, d_out, n, static_cast<uint32_t *>(ctx->d_scratch), total_out, &launches));
+    ctx->launches += uint64_t(launches);
     return SPHX_OK;
 }
 
 size_t scan_scratch_entries(size_t n) { return (n + kScanTile - 1) / kScanTile + 1; }
 
-// The same three passes on a stream with caller-owned tile scratch of
-// scan_scratch_entries(n) entries; enqueues only (no allocation, no synchronisation), so a
-// stream capture may record it.
-int exclusive_scan_into(cudaStream_t s, const uint32_t *d_in, uint32_t *d_out, size_t n, uint32_t *tiles)
+// The same passes on a stream with caller-owned tile scratch of scan_scratch_entries(n)
+// entries; enqueues only (no allocation, no synchronisation), so a stream capture may record it.
+int exclusive_scan_into(cudaStream_t s, const uint32_t *d_in, uint32_t *d_out, size_t n, uint32_t *tiles,
+                        uint32_t *total_out)
 {
-    if (n == 0)
-        return SPHX_OK;
-    size_t ntiles = (n + kScanTile - 1) / kScanTile;
-    k_scan_tile_sums<<<unsigned(ntiles), kBlock, 0, s>>>(d_in, n, tiles);
-    SPHX_CUDA(cudaGetLastError());
-    k_scan_tile_prefix<<<1, 1024, 0, s>>>(tiles, ntiles, tiles + ntiles);
-    SPHX_CUDA(cudaGetLastError());
-    k_scan_apply<<<unsigned(ntiles), kBlock, 0, s>>>(d_in, d_out, n, tiles);
-    SPHX_CUDA(cudaGetLastError());
-    return SPHX_OK;
+    int launches = 0;
+    return n == 0 ? SPHX_OK : scan_passes(s, d_in, d_out, n, tiles, total_out, &launches);
 }
 
 // Stable counting sort of n keys in [0, nkeys): d_offset[nkeys+1] gets the key offsets,
@@ -389,9 +418,7 @@ int counting_sort_by_key(sphx_ctx ctx, const uint32_t *d_key, size_t n, uint32_t
     }
     k_count_keys<<<grid_for(n, kBlock), kBlock, 0, s>>>(n, d_key, d_rank, d_count);
     SPHX_LAUNCHED(ctx);
-    SPHX_TRY(exclusive_scan(ctx, d_count, d_offset, nkeys));
-    k_set_total<<<1, 1, 0, s>>>(d_offset, nkeys, uint32_t(n));
-    SPHX_LAUNCHED(ctx);
+    SPHX_TRY(exclusive_scan(ctx, d_count, d_offset, nkeys, d_offset + nkeys));
     k_scatter<<<grid_for(n, kBlock), kBlock, 0, s>>>(n, d_key, d_rank, d_offset, d_perm);
     SPHX_LAUNCHED(ctx);
     k_sort_segments<<<grid_for(nkeys, kBlock), kBlock, 0, s>>>(nkeys, d_offset, d_perm);
@@ -411,8 +438,8 @@ int sphx_cell_list_s::reserve_entries(size_t ne, size_t keep)
     uint32_t *idx = nullptr, *flag = nullptr, *scan = nullptr, *perm = nullptr;
     SPHX_CUDA(cudaMalloc(&pos, 3 * cap * sizeof(double)));
     SPHX_CUDA(cudaMalloc(&idx, cap * sizeof(uint32_t)));
-    SPHX_CUDA(cudaMalloc(&flag, cap * sizeof(uint32_t)));
-    SPHX_CUDA(cudaMalloc(&scan, cap * sizeof(uint32_t)));
+    SPHX_CUDA(cudaMalloc(&flag, 2 * cap * sizeof(uint32_t))); // both sides of an axis
+    SPHX_CUDA(cudaMalloc(&scan, 2 * cap * sizeof(uint32_t)));
     SPHX_CUDA(cudaMalloc(&perm, cap * sizeof(uint32_t)));
     if (keep && entry_pos)
     {
@@ -535,41 +562,33 @@ int update_periodic(sphx_cell_list cl, sphx_body body, const double *pos)
     {
         if (!(cl->periodic_mask & (1 << a)))
             continue;
-        double lo = cl->per_lower[a], up = cl->per_upper[a], rc = cl->per_cutoff, L = up - lo;
-        size_t n_axis = n_cur; // the entries this axis images (both sides)
-        for (int side = 0; side < 2; ++side)
+        const double lo = cl->per_lower[a], up = cl->per_upper[a], rc = cl->per_cutoff;
+        if (n_cur == 0)
+            break;
+        k_image_flags<<<grid_for(n_cur, kBlock), kBlock, 0, s>>>(n_cur, cl->entry_cap, cl->entry_pos, a, lo, up, rc,
+                                                                 cl->entry_flag);
+        SPHX_LAUNCHED(ctx);
+        uint32_t *d_total = reinterpret_cast<uint32_t *>(ctx->d_red);
+        SPHX_TRY(exclusive_scan(ctx, cl->entry_flag, cl->entry_scan, 2 * n_cur, d_total));
+        SPHX_CUDA(cudaMemcpyAsync(ctx->h_red, d_total, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+        SPHX_CUDA(cudaStreamSynchronize(s));
+        const size_t total = *reinterpret_cast<const uint32_t *>(ctx->h_red);
+        if (total == 0)
+            continue;
+        if (n_cur + total > cl->entry_cap)
         {
-            if (n_axis == 0)
-                break;
-            double band_lo = side == 0 ? lo : up - rc, band_hi = side == 0 ? lo + rc : up;
-            k_image_flags<<<grid_for(n_axis, kBlock), kBlock, 0, s>>>(n_axis, cl->entry_cap, cl->entry_pos, a,
-                                                                       band_lo, band_hi, cl->entry_flag);
+            // regrowth keeps the entries generated so far; flags and scan are recomputed
+            SPHX_TRY(cl->reserve_entries(n_cur + total, n_cur));
+            k_image_flags<<<grid_for(n_cur, kBlock), kBlock, 0, s>>>(n_cur, cl->entry_cap, cl->entry_pos, a, lo, up,
+                                                                     rc, cl->entry_flag);
             SPHX_LAUNCHED(ctx);
-            uint32_t total = 0;
-            SPHX_TRY(exclusive_scan(ctx, cl->entry_flag, cl->entry_scan, n_axis));
-            // total = last scan value + last flag
-            uint32_t last[2] = {0, 0};
-            SPHX_CUDA(cudaMemcpyAsync(&last[0], cl->entry_scan + n_axis - 1, 4, cudaMemcpyDeviceToHost, s));
-            SPHX_CUDA(cudaMemcpyAsync(&last[1], cl->entry_flag + n_axis - 1, 4, cudaMemcpyDeviceToHost, s));
-            SPHX_CUDA(cudaStreamSynchronize(s));
-            total = last[0] + last[1];
-            if (total == 0)
-                continue;
-            if (n_cur + total > cl->entry_cap)
-            {
-                // regrowth keeps the entries generated so far; flags and scan are recomputed
-                SPHX_TRY(cl->reserve_entries(n_cur + total, n_cur));
-                k_image_flags<<<grid_for(n_axis, kBlock), kBlock, 0, s>>>(n_axis, cl->entry_cap, cl->entry_pos, a,
-                                                                           band_lo, band_hi, cl->entry_flag);
-                SPHX_LAUNCHED(ctx);
-                SPHX_TRY(exclusive_scan(ctx, cl->entry_flag, cl->entry_scan, n_axis));
-            }
-            k_image_emit<<<grid_for(n_axis, kBlock), kBlock, 0, s>>>(n_axis, D, cl->entry_cap, cl->entry_pos,
-                                                                      cl->entry_idx, cl->entry_flag, cl->entry_scan,
-                                                                      n_cur, a, side == 0 ? L : -L);
-            SPHX_LAUNCHED(ctx);
-            n_cur += total;
+            SPHX_TRY(exclusive_scan(ctx, cl->entry_flag, cl->entry_scan, 2 * n_cur));
         }
+        k_image_emit<<<grid_for(2 * n_cur, kBlock), kBlock, 0, s>>>(n_cur, D, cl->entry_cap, cl->entry_pos,
+                                                                    cl->entry_idx, cl->entry_flag, cl->entry_scan, a,
+                                                                    up - lo);
+        SPHX_LAUNCHED(ctx);
+        n_cur += total;
     }
     size_t ne = n_cur;
     SPHX_TRY(cl->reserve(ne));
@@ -587,9 +606,7 @@ int update_periodic(sphx_cell_list cl, sphx_body body, const double *pos)
                                                                     cl->rank, cl->cell_count);
         SPHX_LAUNCHED(ctx);
     }
-    SPHX_TRY(exclusive_scan(ctx, cl->cell_count, cl->cell_offset, cl->ncells));
-    k_set_total<<<1, 1, 0, s>>>(cl->cell_offset, uint32_t(cl->ncells), uint32_t(ne));
-    SPHX_LAUNCHED(ctx);
+    SPHX_TRY(exclusive_scan(ctx, cl->cell_count, cl->cell_offset, cl->ncells, cl->cell_offset + cl->ncells));
     if (ne == 0)
         return SPHX_OK;
     if (cl->entry_cap < ne)
@@ -678,9 +695,7 @@ extern "C" int sphx_cell_list_update(sphx_cell_list cl, sphx_body body)
             k_hash_count<3><<<grid_for(n, kBlock), kBlock, 0, s>>>(n, p, m, cl->cell_of, cl->rank, cl->cell_count);
         SPHX_LAUNCHED(ctx);
     }
-    SPHX_TRY(exclusive_scan(ctx, cl->cell_count, cl->cell_offset, cl->ncells));
-    k_set_total<<<1, 1, 0, s>>>(cl->cell_offset, uint32_t(cl->ncells), uint32_t(n));
-    SPHX_LAUNCHED(ctx);
+    SPHX_TRY(exclusive_scan(ctx, cl->cell_count, cl->cell_offset, cl->ncells, cl->cell_offset + cl->ncells));
     if (n == 0)
         return SPHX_OK;
     k_scatter<<<grid_for(n, kBlock), kBlock, 0, s>>>(n, cl->cell_of, cl->rank, cl->cell_offset, cl->particle_index);
@@ -909,7 +924,7 @@ extern "C" int sphx_exclusive_scan_u32_noalloc(void *stream, const uint32_t *d_i
     SPHX_CUDA(cudaGetLastError());
     k_scan_tile_prefix<<<1, 1024, 0, s>>>(tiles, ntiles, tiles + ntiles);
     SPHX_CUDA(cudaGetLastError());
-    k_scan_apply<<<unsigned(ntiles), kBlock, 0, s>>>(d_in, d_out, n, tiles);
+    k_scan_apply<true><<<unsigned(ntiles), kBlock, 0, s>>>(d_in, d_out, n, tiles, nullptr);
     SPHX_CUDA(cudaGetLastError());
     if (total)
     {

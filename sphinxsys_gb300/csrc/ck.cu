@@ -647,19 +647,6 @@ __global__ void __launch_bounds__(kBlock) k_ck_second(size_t n, CKFluid f, CKWal
     f.rho[i] = comp * k.rho0;
 }
 
-__device__ __forceinline__ void block_max(unsigned long long *slot, double v)
-{
-    unsigned long long b = ordered_bits(v);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1)
-    {
-        unsigned long long y = __shfl_down_sync(0xffffffffu, b, o);
-        b = y > b ? y : b;
-    }
-    if ((threadIdx.x & 31u) == 0)
-        atomicMax(slot, b);
-}
-
 // FreeSurfaceIndicationCK<Inner<WithUpdate>, Contact<>> (surface_indication_ck.hpp:49-150):
 // position divergence -sum dW V r over the inner neighbours with the spatial-temporal rule
 // (a particle below the threshold that was not a surface particle and has no previous
@@ -755,7 +742,7 @@ __global__ void k_ck_indication_update(size_t n, CKFluid f, Lists in, const doub
 }
 
 template <int D>
-__global__ void k_ck_acoustic_max(size_t n, CKFluid f, double c0, double h_min, unsigned long long *slot)
+__global__ void k_ck_acoustic_max(size_t n, CKFluid f, double c0, double h_min, MaxSlot slot)
 {
     double m = 0.0;
     for (size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += size_t(gridDim.x) * blockDim.x)
@@ -769,11 +756,11 @@ __global__ void k_ck_acoustic_max(size_t n, CKFluid f, double c0, double h_min, 
         double acc_scale = sqrt(4.0 * h_min * sqrt(dot<D>(F, F)) / f.mass[i]);
         m = fmax(m, fmax(c0 + sqrt(dot<D>(v, v)), acc_scale));
     }
-    block_max(slot, m);
+    block_max_to(slot, m);
 }
 
 template <int D>
-__global__ void k_ck_advection_max(size_t n, CKFluid f, unsigned long long *slot)
+__global__ void k_ck_advection_max(size_t n, CKFluid f, MaxSlot slot)
 {
     double m = 0.0;
     for (size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += size_t(gridDim.x) * blockDim.x)
@@ -783,7 +770,7 @@ __global__ void k_ck_advection_max(size_t n, CKFluid f, unsigned long long *slot
             v[a] = f.vel[a * n + i];
         m = fmax(m, dot<D>(v, v));
     }
-    block_max(slot, m);
+    block_max_to(slot, m);
 }
 
 template <int D, int LANES>
@@ -929,10 +916,8 @@ unsigned red_grid(sphx_ctx ctx, size_t n)
 
 int read_max(sphx_ctx ctx, double *out)
 {
-    SPHX_CUDA(cudaMemcpyAsync(ctx->h_red, ctx->d_red, sizeof(unsigned long long), cudaMemcpyDeviceToHost,
-                              ctx->stream));
     SPHX_CUDA(cudaStreamSynchronize(ctx->stream));
-    *out = from_ordered_bits(ctx->h_red[0]);
+    *out = from_ordered_bits(*max_slot(ctx).out);
     return SPHX_OK;
 }
 
@@ -1155,13 +1140,11 @@ extern "C" int sphx_ck_acoustic_time_step(sphx_body b, const sphx_fluid_params *
     CKFluid f;
     SPHX_TRY(ck_fluid(b, f));
     sphx_ctx ctx = b->ctx;
-    SPHX_CUDA(cudaMemsetAsync(ctx->d_red, 0, sizeof(unsigned long long), ctx->stream));
     if (b->n > 0)
-        CK_DISPATCH(b, k_ck_acoustic_max, red_grid(ctx, b->n), b->n, f, p->c0, p->h, ctx->d_red);
+        CK_DISPATCH(b, k_ck_acoustic_max, red_grid(ctx, b->n), b->n, f, p->c0, p->h, max_slot(ctx));
     double m = 0;
-    SPHX_TRY(read_max(ctx, &m));
-    if (b->n == 0)
-        m = 0.0;
+    if (b->n > 0)
+        SPHX_TRY(read_max(ctx, &m));
     *dt = p->acoustic_cfl * p->h / (m + kTinyReal);
     return SPHX_OK;
 }
@@ -1173,13 +1156,11 @@ extern "C" int sphx_ck_advection_time_step(sphx_body b, const sphx_fluid_params 
     CKFluid f;
     SPHX_TRY(ck_fluid(b, f));
     sphx_ctx ctx = b->ctx;
-    SPHX_CUDA(cudaMemsetAsync(ctx->d_red, 0, sizeof(unsigned long long), ctx->stream));
     if (b->n > 0)
-        CK_DISPATCH(b, k_ck_advection_max, red_grid(ctx, b->n), b->n, f, ctx->d_red);
+        CK_DISPATCH(b, k_ck_advection_max, red_grid(ctx, b->n), b->n, f, max_slot(ctx));
     double m = 0;
-    SPHX_TRY(read_max(ctx, &m));
-    if (b->n == 0)
-        m = 0.0;
+    if (b->n > 0)
+        SPHX_TRY(read_max(ctx, &m));
     *dt = p->advection_cfl * p->h / (std::max(std::sqrt(m), p->U_ref) + kTinyReal);
     return SPHX_OK;
 }

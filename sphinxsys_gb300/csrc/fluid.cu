@@ -752,36 +752,8 @@ __global__ void __launch_bounds__(kBlock, kBlocks2)
 // ---------------------------------------------------------------- reductions
 // Max reductions write the order-preserving bits of non-negative doubles; the warp and
 // block maxima are exact, so the result does not depend on the launch order.
-__device__ __forceinline__ void block_max_to(unsigned long long *slot, double v)
-{
-    unsigned long long b = ordered_bits(v);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1)
-    {
-        unsigned long long y = __shfl_down_sync(0xffffffffu, b, o);
-        b = y > b ? y : b;
-    }
-    __shared__ unsigned long long sm[32];
-    unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-    if (lane == 0)
-        sm[warp] = b;
-    __syncthreads();
-    if (warp == 0)
-    {
-        b = lane < (blockDim.x >> 5) ? sm[lane] : 0ull;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1)
-        {
-            unsigned long long y = __shfl_down_sync(0xffffffffu, b, o);
-            b = y > b ? y : b;
-        }
-        if (lane == 0)
-            atomicMax(slot, b);
-    }
-}
-
 template <int D>
-__global__ void k_acoustic_max(size_t n, const double *__restrict__ vel, double c0, unsigned long long *slot)
+__global__ void k_acoustic_max(size_t n, const double *__restrict__ vel, double c0, MaxSlot slot)
 {
     double m = -1.0;
     for (size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += size_t(gridDim.x) * blockDim.x)
@@ -798,7 +770,7 @@ __global__ void k_acoustic_max(size_t n, const double *__restrict__ vel, double 
 template <int D>
 __global__ void k_advection_max(size_t n, const double *__restrict__ vel, const double *__restrict__ force,
                                 const double *__restrict__ fprior, const double *__restrict__ mass, double h_min,
-                                unsigned long long *slot)
+                                MaxSlot slot)
 {
     double m = -1.0e300;
     for (size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += size_t(gridDim.x) * blockDim.x)
@@ -902,7 +874,7 @@ __global__ void k_sum_partials(unsigned np, const double *__restrict__ partials,
 
 template <int D>
 __global__ void k_upper_front(size_t n, const double *__restrict__ pos, int axis, double l0, double l1, double l2,
-                              double u0, double u1, double u2, unsigned long long *slot)
+                              double u0, double u1, double u2, MaxSlot slot)
 {
     double lo[3] = {l0, l1, l2}, up[3] = {u0, u1, u2};
     double m = -1.0e300;
@@ -979,23 +951,25 @@ int check_pair(sphx_relation inner, sphx_relation wall, const sphx_fluid_params 
 
 int read_max(sphx_ctx ctx, double *out)
 {
-    SPHX_CUDA(cudaMemcpyAsync(ctx->h_red, ctx->d_red, sizeof(unsigned long long), cudaMemcpyDeviceToHost,
-                              ctx->stream));
     SPHX_CUDA(cudaStreamSynchronize(ctx->stream));
-    *out = from_ordered_bits(ctx->h_red[0]);
+    *out = from_ordered_bits(*max_slot(ctx).out);
     return SPHX_OK;
 }
 
 // ViscousForce<Inner<>, FixedViscosity, NoKernelCorrection> (viscous_dynamics.hpp:25-53) and
 // the ForcePrior update (force_prior.hpp:22-26): the configuration-time r, e, dW of the inner
-// relation, e . (2 e) for the (absent) kernel correction.
-template <int D>
-__global__ void __launch_bounds__(kBlock) k_viscous_inner(size_t n, InnerPairs in, const double *__restrict__ R, const double *__restrict__ vel,
+// relation, e . (2 e) = 2 for the (absent) kernel correction.  One division a pair; LANES
+// threads share a particle.
+template <int D, int LANES>
+__global__ void __launch_bounds__(kBlock) k_viscous_inner(size_t n, InnerPairs in, const double *__restrict__ R,
+                                                          const double *__restrict__ vel,
                                                           const double *__restrict__ Vol, double mu, double h,
                                                           double *__restrict__ viscous, double *__restrict__ prev,
                                                           double *__restrict__ force_prior)
 {
-    size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
+    const size_t g = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
+    const size_t i = g / LANES;
+    const unsigned sub = unsigned(g % LANES);
     if (i >= n)
         return;
     double f[3] = {0, 0, 0}, vi[3] = {0, 0, 0};
@@ -1003,35 +977,27 @@ __global__ void __launch_bounds__(kBlock) k_viscous_inner(size_t n, InnerPairs i
     for (int a = 0; a < D; ++a)
         vi[a] = vel[a * n + i];
     const unsigned cnt = min(in.count[i], in.cap);
-    for (unsigned s = 0; s < cnt; ++s)
+    for (unsigned s = sub; s < cnt; s += LANES)
     {
-        size_t slot = size_t(s) * n + i;
-        uint32_t j = in.J[slot];
+        const size_t slot = size_t(s) * n + i;
+        const uint32_t j = in.J[slot];
         if (!entry_ok(in, j))
             continue;
-        const fx::Entry<D> q = in.at.load<D>(slot);
-        double e[3] = {0, 0, 0};
+        const double c = fx::decode(in.at.load<D>(slot).k) * Vol[j] / (R[slot] + 0.01 * h);
 #pragma unroll
         for (int a = 0; a < D; ++a)
-            e[a] = fx::decode(q.e[a]);
-        double ee = 0;
-#pragma unroll
-        for (int a = 0; a < D; ++a)
-            ee += e[a] * (2.0 * e[a]);
-        double denom = R[slot] + 0.01 * h;
-        double dWV_factor = in.factor * fx::decode(q.k);
-#pragma unroll
-        for (int a = 0; a < D; ++a)
-        {
-            double vd = (vi[a] - vel[a * n + j]) / denom;
-            f[a] += ee * mu * vd * dWV_factor * Vol[j];
-        }
+            f[a] = fma(c, vi[a] - vel[a * n + j], f[a]);
     }
-    const double Vol_i = Vol[i];
+#pragma unroll
+    for (int a = 0; a < D; ++a)
+        f[a] = fx::group_sum<LANES>(f[a]);
+    if (sub != 0)
+        return;
+    const double scale = 2.0 * mu * in.factor * Vol[i];
 #pragma unroll
     for (int a = 0; a < D; ++a)
     {
-        double v = f[a] * Vol_i;
+        const double v = f[a] * scale;
         force_prior[a * n + i] += v - prev[a * n + i];
         prev[a * n + i] = v;
         viscous[a * n + i] = v;
@@ -1042,34 +1008,42 @@ __global__ void __launch_bounds__(kBlock) k_viscous_inner(size_t n, InnerPairs i
 // .hpp:32-66): kernel-gradient integral from the configuration-time dW, e, then the position
 // shift with the limiter min(100 h^2 |.|^2, 1); interaction and update fused (the update
 // moves only the particle's own position, which no neighbour term reads).
-template <int D>
+template <int D, int LANES>
 __global__ void __launch_bounds__(kBlock) k_tvc_inner(size_t n, InnerPairs in, const double *__restrict__ Vol,
                                                       double h2, double scaling, double *__restrict__ pos)
 {
-    size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
+    const size_t g = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
+    const size_t i = g / LANES;
+    const unsigned sub = unsigned(g % LANES);
     if (i >= n)
         return;
     double inc[3] = {0, 0, 0};
     const unsigned cnt = min(in.count[i], in.cap);
-    for (unsigned s = 0; s < cnt; ++s)
+    for (unsigned s = sub; s < cnt; s += LANES)
     {
-        size_t slot = size_t(s) * n + i;
-        uint32_t j = in.J[slot];
+        const size_t slot = size_t(s) * n + i;
+        const uint32_t j = in.J[slot];
         if (!entry_ok(in, j))
             continue;
         const fx::Entry<D> q = in.at.load<D>(slot);
-        double w = (1.0 + 1.0) * in.factor * fx::decode(q.k) * Vol[j];
+        const double w = fx::decode(q.k) * Vol[j];
 #pragma unroll
         for (int a = 0; a < D; ++a)
-            inc[a] -= w * fx::decode(q.e[a]);
+            inc[a] = fma(w, fx::decode(q.e[a]), inc[a]);
     }
-    double sq = inc[0] * inc[0] + inc[1] * inc[1];
-    if (D == 3)
-        sq = sq + inc[2] * inc[2];
+    double sq = 0.0;
+#pragma unroll
+    for (int a = 0; a < D; ++a)
+    {
+        inc[a] = -2.0 * in.factor * fx::group_sum<LANES>(inc[a]);
+        sq = fma(inc[a], inc[a], sq);
+    }
+    if (sub != 0)
+        return;
     double lim = fmin(100.0 * (h2 * sq), 1.0);
 #pragma unroll
     for (int a = 0; a < D; ++a)
-        pos[a * n + i] += scaling * lim * inc[a] * 1.0 * 1.0;
+        pos[a * n + i] += scaling * lim * inc[a];
 }
 
 // The particle values of a sweep (half 0: pressures, half 1: velocities) in the relation's
@@ -1247,22 +1221,20 @@ extern "C" int sphx_acoustic_time_step(sphx_body b, const sphx_fluid_params *p, 
     SPHX_TRY(b->require("Velocity", SPHX_F64, b->dim, &vel));
     sphx_ctx ctx = b->ctx;
     size_t n = b->n;
-    SPHX_CUDA(cudaMemsetAsync(ctx->d_red, 0, sizeof(unsigned long long), ctx->stream));
     if (n > 0)
     {
         unsigned g = reduce_grid(ctx, n);
         if (b->dim == 2)
             k_acoustic_max<2><<<g, kBlock, 0, ctx->stream>>>(n, static_cast<const double *>(vel->dev), p->c0,
-                                                             ctx->d_red);
+                                                             max_slot(ctx));
         else
             k_acoustic_max<3><<<g, kBlock, 0, ctx->stream>>>(n, static_cast<const double *>(vel->dev), p->c0,
-                                                             ctx->d_red);
+                                                             max_slot(ctx));
         SPHX_LAUNCHED(ctx);
     }
-    double m;
-    SPHX_TRY(read_max(ctx, &m));
-    if (n == 0)
-        m = -1.79769313486231570815e308; // ReduceMax initial value MinReal
+    double m = -1.79769313486231570815e308; // ReduceMax initial value MinReal
+    if (n > 0)
+        SPHX_TRY(read_max(ctx, &m));
     *dt = p->acoustic_cfl * p->h / (m + kTinyReal);
     return SPHX_OK;
 }
@@ -1275,20 +1247,20 @@ extern "C" int sphx_advection_time_step(sphx_body b, const sphx_fluid_params *p,
     SPHX_TRY(fluid_vars(b, f));
     sphx_ctx ctx = b->ctx;
     size_t n = b->n;
-    SPHX_CUDA(cudaMemsetAsync(ctx->d_red, 0, sizeof(unsigned long long), ctx->stream));
     if (n > 0)
     {
         unsigned g = reduce_grid(ctx, n);
         if (b->dim == 2)
             k_advection_max<2><<<g, kBlock, 0, ctx->stream>>>(n, f.vel, f.force, f.force_prior, f.mass, p->h,
-                                                              ctx->d_red);
+                                                              max_slot(ctx));
         else
             k_advection_max<3><<<g, kBlock, 0, ctx->stream>>>(n, f.vel, f.force, f.force_prior, f.mass, p->h,
-                                                              ctx->d_red);
+                                                              max_slot(ctx));
         SPHX_LAUNCHED(ctx);
     }
-    double m;
-    SPHX_TRY(read_max(ctx, &m));
+    double m = 0.0;
+    if (n > 0)
+        SPHX_TRY(read_max(ctx, &m));
     double speed_max = n > 0 ? sqrt(m) : 0.0;
     *dt = p->advection_cfl * p->h / (std::max(speed_max, p->U_ref) + kTinyReal);
     return SPHX_OK;
@@ -1407,13 +1379,7 @@ extern "C" int sphx_viscous_force_inner(sphx_relation inner, double mu)
     sphx_ctx ctx = b->ctx;
     const InnerPairs in = pairs_of(inner);
     auto d = [](Field *f) { return static_cast<double *>(f->dev); };
-    if (D == 2)
-        k_viscous_inner<2><<<grid_for(n, kBlock), kBlock, 0, ctx->stream>>>(n, in, inner->r, d(vel), d(Vol), mu, inner->h,
-                                                                            d(visc), d(prev), d(fp));
-    else
-        k_viscous_inner<3><<<grid_for(n, kBlock), kBlock, 0, ctx->stream>>>(n, in, inner->r, d(vel), d(Vol), mu, inner->h,
-                                                                            d(visc), d(prev), d(fp));
-    SPHX_LAUNCHED(ctx);
+    SWEEP_DISPATCH(k_viscous_inner, D, ctx, n, n, in, inner->r, d(vel), d(Vol), mu, inner->h, d(visc), d(prev), d(fp));
     return SPHX_OK;
 }
 
@@ -1436,11 +1402,7 @@ extern "C" int sphx_transport_velocity_correction_inner(sphx_relation inner, dou
     const InnerPairs in = pairs_of(inner);
     double *p = static_cast<double *>(pos->dev);
     const double *V = static_cast<const double *>(Vol->dev);
-    if (D == 2)
-        k_tvc_inner<2><<<grid_for(n, kBlock), kBlock, 0, ctx->stream>>>(n, in, V, h2, coefficient * h2, p);
-    else
-        k_tvc_inner<3><<<grid_for(n, kBlock), kBlock, 0, ctx->stream>>>(n, in, V, h2, coefficient * h2, p);
-    SPHX_LAUNCHED(ctx);
+    SWEEP_DISPATCH(k_tvc_inner, D, ctx, n, n, in, V, h2, coefficient * h2, p);
     return SPHX_OK;
 }
 
@@ -1452,21 +1414,21 @@ extern "C" int sphx_maximum_speed(sphx_body b, double *out)
     SPHX_TRY(b->require("Velocity", SPHX_F64, b->dim, &vel));
     sphx_ctx ctx = b->ctx;
     size_t n = b->n;
-    SPHX_CUDA(cudaMemsetAsync(ctx->d_red, 0, sizeof(unsigned long long), ctx->stream));
     if (n > 0)
     {
         unsigned g = reduce_grid(ctx, n);
         if (b->dim == 2)
             k_acoustic_max<2><<<g, kBlock, 0, ctx->stream>>>(n, static_cast<const double *>(vel->dev), 0.0,
-                                                             ctx->d_red);
+                                                             max_slot(ctx));
         else
             k_acoustic_max<3><<<g, kBlock, 0, ctx->stream>>>(n, static_cast<const double *>(vel->dev), 0.0,
-                                                             ctx->d_red);
+                                                             max_slot(ctx));
         SPHX_LAUNCHED(ctx);
     }
     double m = 0;
-    SPHX_TRY(read_max(ctx, &m));
-    *out = n > 0 ? m : 0.0;
+    if (n > 0)
+        SPHX_TRY(read_max(ctx, &m));
+    *out = m;
     return SPHX_OK;
 }
 
@@ -1479,19 +1441,20 @@ extern "C" int sphx_upper_front_in_axis_direction(sphx_body b, int axis, const d
     SPHX_TRY(b->need("Position", SPHX_F64, b->dim, &pos));
     sphx_ctx ctx = b->ctx;
     size_t n = b->n;
-    SPHX_CUDA(cudaMemsetAsync(ctx->d_red, 0, sizeof(unsigned long long), ctx->stream));
     if (n > 0)
     {
         unsigned g = reduce_grid(ctx, n);
         double l2 = b->dim == 3 ? lo[2] : 0.0, u2 = b->dim == 3 ? up[2] : 0.0;
         if (b->dim == 2)
             k_upper_front<2><<<g, kBlock, 0, ctx->stream>>>(n, static_cast<const double *>(pos->dev), axis, lo[0],
-                                                            lo[1], l2, up[0], up[1], u2, ctx->d_red);
+                                                            lo[1], l2, up[0], up[1], u2, max_slot(ctx));
         else
             k_upper_front<3><<<g, kBlock, 0, ctx->stream>>>(n, static_cast<const double *>(pos->dev), axis, lo[0],
-                                                            lo[1], l2, up[0], up[1], u2, ctx->d_red);
+                                                            lo[1], l2, up[0], up[1], u2, max_slot(ctx));
         SPHX_LAUNCHED(ctx);
     }
-    SPHX_TRY(read_max(ctx, front));
+    *front = from_ordered_bits(0);
+    if (n > 0)
+        SPHX_TRY(read_max(ctx, front));
     return SPHX_OK;
 }

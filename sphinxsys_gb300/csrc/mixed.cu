@@ -143,8 +143,6 @@ __global__ void k_mp_sort_segments(size_t nseg, const uint32_t *__restrict__ off
         sort_segment(idx, offset[c], offset[c + 1]);
 }
 
-__global__ void k_mp_set_total(uint32_t *offset, size_t ncells, uint32_t total) { offset[ncells] = total; }
-
 // Gathers the state into the new cell order.
 template <int D>
 __global__ void k_mp_gather(size_t n, const uint32_t *__restrict__ perm, const uint32_t *__restrict__ ncell,
@@ -1266,9 +1264,7 @@ int sort_keys(sphx_mp mp, size_t n, uint32_t *offset)
 {
     sphx_ctx ctx = mp->ctx;
     cudaStream_t s = ctx->stream;
-    SPHX_TRY(exclusive_scan(ctx, mp->count, offset, mp->ncells));
-    k_mp_set_total<<<1, 1, 0, s>>>(offset, mp->ncells, uint32_t(n));
-    SPHX_LAUNCHED(ctx);
+    SPHX_TRY(exclusive_scan(ctx, mp->count, offset, mp->ncells, offset + mp->ncells));
     if (n == 0)
         return SPHX_OK;
     k_mp_scatter<<<grid_for(n, 256), 256, 0, s>>>(n, mp->key, mp->rank, offset, mp->perm);
@@ -1308,9 +1304,7 @@ int tile_order(sphx_mp mp)
     SPHX_CUDA(cudaMemsetAsync(mp->count, 0, nt * sizeof(uint32_t), s));
     k_mp_tile_key<D><<<grid_for(n, 256), 256, 0, s>>>(n, mp->a.geo0, ts, mp->key, mp->rank, mp->count);
     SPHX_LAUNCHED(ctx);
-    SPHX_TRY(exclusive_scan(ctx, mp->count, mp->tile_offset, nt));
-    k_mp_set_total<<<1, 1, 0, s>>>(mp->tile_offset, nt, uint32_t(n));
-    SPHX_LAUNCHED(ctx);
+    SPHX_TRY(exclusive_scan(ctx, mp->count, mp->tile_offset, nt, mp->tile_offset + nt));
     k_mp_scatter<<<grid_for(n, 256), 256, 0, s>>>(n, mp->key, mp->rank, mp->tile_offset, mp->order);
     SPHX_LAUNCHED(ctx);
     k_mp_sort_segments<<<grid_for(nt, 256), 256, 0, s>>>(nt, mp->tile_offset, mp->order);

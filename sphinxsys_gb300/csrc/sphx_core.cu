@@ -179,6 +179,7 @@ extern "C" int sphx_ctx_create(int device, void *stream, sphx_ctx *out)
     }
     SPHX_CUDA(cudaMalloc(&c->d_red, 64 * sizeof(unsigned long long)));
     SPHX_CUDA(cudaMallocHost(&c->h_red, 64 * sizeof(unsigned long long)));
+    SPHX_CUDA(cudaMemsetAsync(c->d_red, 0, 64 * sizeof(unsigned long long), c->stream));
     *out = c;
     return SPHX_OK;
 }

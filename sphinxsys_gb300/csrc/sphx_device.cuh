@@ -86,6 +86,41 @@ __host__ __device__ __forceinline__ double from_ordered_bits(unsigned long long 
     return d;
 }
 
+// Maximum over a grid, delivered by the grid itself: the block maximum goes to *slot, and the
+// last block to finish hands the result to the host word `out` (pinned) and leaves slot and
+// counter zero for the next call, so a reduction is one launch and one wait.
+struct MaxSlot
+{
+    unsigned long long *slot, *counter, *out;
+};
+inline MaxSlot max_slot(sphx_ctx ctx) { return MaxSlot{ctx->d_red + 32, ctx->d_red + 33, ctx->h_red + 32}; }
+__device__ __forceinline__ void block_max_to(const MaxSlot &m, double v)
+{
+    unsigned long long b = ordered_bits(v);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+    {
+        unsigned long long y = __shfl_down_sync(0xffffffffu, b, o);
+        b = y > b ? y : b;
+    }
+    __shared__ unsigned long long sm[32];
+    unsigned lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    if (lane == 0)
+        sm[warp] = b;
+    __syncthreads();
+    if (threadIdx.x != 0)
+        return;
+    for (unsigned w = 1; w < (blockDim.x >> 5); ++w)
+        b = sm[w] > b ? sm[w] : b;
+    atomicMax(m.slot, b);
+    __threadfence();
+    if (atomicAdd(m.counter, 1ull) != gridDim.x - 1)
+        return;
+    *m.out = atomicExch(m.slot, 0ull);
+    *m.counter = 0;
+    __threadfence_system();
+}
+
 // atomicMax of v over the lanes that reach this call together: one atomic per group of
 // converged lanes instead of one per lane on a single contended address.
 __device__ __forceinline__ void warp_atomic_max(unsigned int *addr, unsigned int v)
