@@ -310,10 +310,107 @@ __device__ __forceinline__ void for_batches(const InnerPairs &in, size_t n, size
     }
 }
 
+// Whether a sweep sums the wall terms itself: with the most threads per particle (few
+// particles) one launch less is worth more than the lanes that idle (2D, 3,200 particles:
+// 449 us a step against 486); else they come from k_wall (3D, 46,000 particles: 1,362 us
+// against 1,597).
+template <int D, int LANES>
+__host__ __device__ constexpr bool walls_in_sweep()
+{
+    return LANES == (D == 2 ? 4 : 8);
+}
+
+// The sums of one particle over its list: fixed point with the alignment a of the force, or
+// (general path) doubles in the words of hh.
+template <int D>
+struct SweepSums
+{
+    fx::Sum force[D], rate;
+    int a = 0;
+    double wall[D + 1]; // wall terms summed in the sweep (see walls_in_sweep)
+    __device__ __forceinline__ void set(const double *f, double r)
+    {
+#pragma unroll
+        for (int d = 0; d < D; ++d)
+            force[d].hh = __double_as_longlong(f[d]);
+        rate.hh = __double_as_longlong(r);
+    }
+    __device__ __forceinline__ void get(double *f, double *r) const
+    {
+#pragma unroll
+        for (int d = 0; d < D; ++d)
+            f[d] = __longlong_as_double(force[d].hh);
+        *r = __longlong_as_double(rate.hh);
+    }
+};
+
+// With several threads per particle the sums are handed through shared memory to the block's
+// first threads, one per particle: the FP64 work of a particle then runs with all lanes of
+// its warps busy instead of one in LANES.  Returns whether this thread finishes a particle
+// (i, s become its index and sums).
+template <int D, int LANES>
+__device__ __forceinline__ bool pack_particles(size_t n, unsigned sub, size_t &i, SweepSums<D> &s)
+{
+    if (LANES == 1)
+        return i < n;
+    constexpr bool walls = walls_in_sweep<D, LANES>();
+    constexpr unsigned P = kBlock / LANES, W = (2 * D + 3 + (walls ? D + 1 : 0)) | 1; // odd: no bank conflicts
+    __shared__ long long sm[P * W];
+    if (sub == 0)
+    {
+        long long *q = sm + threadIdx.x / LANES * W;
+#pragma unroll
+        for (int d = 0; d < D; ++d)
+        {
+            q[2 * d] = s.force[d].hh;
+            q[2 * d + 1] = s.force[d].m;
+        }
+        q[2 * D] = s.rate.hh;
+        q[2 * D + 1] = s.rate.m;
+        q[2 * D + 2] = s.a;
+        if (walls)
+#pragma unroll
+            for (int d = 0; d <= D; ++d)
+                q[2 * D + 3 + d] = __double_as_longlong(s.wall[d]);
+    }
+    __syncthreads();
+    i = size_t(blockIdx.x) * P + threadIdx.x;
+    if (threadIdx.x >= P || i >= n)
+        return false;
+    const long long *q = sm + threadIdx.x * W;
+#pragma unroll
+    for (int d = 0; d < D; ++d)
+    {
+        s.force[d].hh = q[2 * d];
+        s.force[d].m = q[2 * d + 1];
+    }
+    s.rate.hh = q[2 * D];
+    s.rate.m = q[2 * D + 1];
+    s.a = int(q[2 * D + 2]);
+    if (walls)
+#pragma unroll
+        for (int d = 0; d <= D; ++d)
+            s.wall[d] = __longlong_as_double(q[2 * D + 3 + d]);
+    return true;
+}
+
+// The wall terms of a particle: from the sweep's own sums or from k_wall.
+template <int D, int LANES>
+__device__ __forceinline__ void add_walls(size_t n, size_t i, const Neighbors &wn, const SweepSums<D> &s,
+                                          const double *__restrict__ wall_sum, double *force, double *rate)
+{
+    if (!wn.count || wn.count[i] == 0)
+        return;
+#pragma unroll
+    for (int d = 0; d < D; ++d)
+        force[d] += walls_in_sweep<D, LANES>() ? s.wall[d] : wall_sum[d * n + i];
+    *rate += walls_in_sweep<D, LANES>() ? s.wall[D] : wall_sum[D * n + i];
+}
+
 // Integration1stHalf in fixed point: F = sum (p_i + p_j) K e and R = sum (p_i - p_j) K.
 template <int D, int LANES>
 __device__ __forceinline__ void fixed_1st(size_t n, size_t i, unsigned sub, const InnerPairs &in,
-                                          const long long *__restrict__ P, double *force, double *diss)
+                                          const long long *__restrict__ P, SweepSums<D> &out)
 {
     constexpr int U = LANES == 1 ? kUnroll1 : 2;
     const long long P_i = P[i];
@@ -371,17 +468,27 @@ __device__ __forceinline__ void fixed_1st(size_t n, size_t i, unsigned sub, cons
                 F[d].fold();
         }
     });
-    const int a = fx::group_min<LANES>(first ? fx::Align::kMost : al.a);
+    out.a = fx::group_min<LANES>(first ? fx::Align::kMost : al.a);
     fx::group_sum<LANES>(R);
-    *diss = R.value() * fx::pow2(32 - fx::kPressureBits - fx::kListBits);
+    out.rate = R;
 #pragma unroll
     for (int d = 0; d < D; ++d)
     {
         if (LANES > 1 && !first)
-            F[d].shift(al.a - a);
+            F[d].shift(al.a - out.a);
         fx::group_sum<LANES>(F[d]);
-        force[d] = F[d].value() * fx::pow2(94 - a - fx::kPressureBits - 2 * fx::kListBits);
+        out.force[d] = F[d];
     }
+}
+// The sums of fixed_1st in units of p0 and of the kernel derivative's prefactor.
+template <int D>
+__device__ __forceinline__ void value_1st(const SweepSums<D> &s, double *force, double *diss)
+{
+    *diss = s.rate.value() * fx::pow2(32 - fx::kPressureBits - fx::kListBits);
+    const double unit = fx::pow2(94 - s.a - fx::kPressureBits - 2 * fx::kListBits);
+#pragma unroll
+    for (int d = 0; d < D; ++d)
+        force[d] = s.force[d].value() * unit;
 }
 
 // A speed of `t` units at alignment 0 in the units of alignment a; 2^57 is above every speed.
@@ -395,8 +502,8 @@ __device__ __forceinline__ long long limit_at(long long t, int a)
 // speed at which the limiter reaches 1.
 template <int D, int LANES>
 __device__ __forceinline__ void fixed_2nd(size_t n, size_t i, unsigned sub, const InnerPairs &in,
-                                          const long long *__restrict__ V, int unit, double u_lim, double *force,
-                                          double *rate)
+                                          const long long *__restrict__ V, int unit, double u_lim,
+                                          SweepSums<D> &out)
 {
     constexpr int U = LANES == 1 ? kUnroll2 : 2;
     const longlong2 *rec = reinterpret_cast<const longlong2 *>(V);
@@ -491,23 +598,34 @@ __device__ __forceinline__ void fixed_2nd(size_t n, size_t i, unsigned sub, cons
                 F[d].fold();
         }
     });
-    const int a = fx::group_min<LANES>(first ? fx::Align::kMost : al.a);
+    out.a = fx::group_min<LANES>(first ? fx::Align::kMost : al.a);
     if (LANES > 1 && !first)
-        R.shift(al.a - a);
+        R.shift(al.a - out.a);
     fx::group_sum<LANES>(R);
-    *rate = R.value() * fx::pow2(120 - a + unit - 2 * fx::kListBits); // 2^57 2^(63 - a)
+    out.rate = R;
 #pragma unroll
     for (int d = 0; d < D; ++d)
     {
         if (LANES > 1 && !first)
         {
-            F[d].shift(al.a - a);
-            F[d].shift(al.a - a);
+            F[d].shift(al.a - out.a);
+            F[d].shift(al.a - out.a);
         }
         fx::group_sum<LANES>(F[d]);
-        // u K: 2^57 2^(63 - a), u: 2^(63 - a), sc: 2^53, the sum: 2^31
-        force[d] = F[d].value() * fx::pow2(126 - 2 * a + 84 + 2 * unit - 3 * fx::kListBits);
+        out.force[d] = F[d];
     }
+}
+// The sums of fixed_2nd: the rate in units of the kernel derivative's prefactor, the force in
+// units of that too.
+template <int D>
+__device__ __forceinline__ void value_2nd(const SweepSums<D> &s, int unit, double *force, double *rate)
+{
+    *rate = s.rate.value() * fx::pow2(120 - s.a + unit - 2 * fx::kListBits); // 2^57 2^(63 - a)
+    // u K: 2^57 2^(63 - a), u: 2^(63 - a), sc: 2^53, the sum: 2^31
+    const double q = fx::pow2(126 - 2 * s.a + 84 + 2 * unit - 3 * fx::kListBits);
+#pragma unroll
+    for (int d = 0; d < D; ++d)
+        force[d] = s.force[d].value() * q;
 }
 
 // The wall terms of particle i, the share of thread `sub` of LANES: Integration1stHalfWithWall
@@ -620,57 +738,56 @@ __global__ void __launch_bounds__(kBlock) k_wall(size_t n, size_t n_active, cons
     sum[D * n + i] = q;
 }
 
-// LANES == 1: the wall terms come from k_wall; else they are summed here.
 template <int D, int LANES>
 __global__ void __launch_bounds__(kBlock, kBlocks1)
-    k_interact_1st(size_t n, FluidVars f, InnerPairs in, Neighbors wn, WallVars w, Riemann rs, Fixed fp, double p0,
-                   double dt, const double *__restrict__ wall_sum)
+    k_interact_1st(size_t n, FluidVars f, InnerPairs in, Neighbors wn, WallVars w, Riemann rs, Fixed fp, double p0, double dt,
+                   const double *__restrict__ wall_sum)
 {
     const size_t g = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    const size_t i = g / LANES;
+    size_t i = g / LANES;
     const unsigned sub = unsigned(g % LANES);
-    if (i >= n)
+    const bool general = !fp.value || __ldcg(fp.flag) == fp.epoch;
+    SweepSums<D> sums;
+    if (i < n)
+    {
+        if (general)
+        {
+            double force[3] = {0, 0, 0}, diss = 0;
+            general_1st<D>(n, i, sub, LANES, f.p, f.Vol, in, force, &diss);
+            diss = fx::group_sum<LANES>(diss);
+#pragma unroll
+            for (int d = 0; d < D; ++d)
+                force[d] = fx::group_sum<LANES>(force[d]);
+            sums.set(force, diss);
+        }
+        else
+            fixed_1st<D, LANES>(n, i, sub, in, fp.value, sums);
+        if (walls_in_sweep<D, LANES>() && wn.count)
+        {
+            double wf[3] = {0, 0, 0}, wr = 0;
+            wall_1st<D, LANES>(n, i, sub, f, wn, w, wf, &wr);
+            sums.wall[D] = fx::group_sum<LANES>(wr);
+#pragma unroll
+            for (int d = 0; d < D; ++d)
+                sums.wall[d] = fx::group_sum<LANES>(wf[d]);
+        }
+    }
+    if (!pack_particles<D, LANES>(n, sub, i, sums))
         return;
     double force[3] = {0, 0, 0};
     double rho_dissipation = 0;
-    if (!fp.value || __ldcg(fp.flag) == fp.epoch)
-    {
-        general_1st<D>(n, i, sub, LANES, f.p, f.Vol, in, force, &rho_dissipation);
-        rho_dissipation = fx::group_sum<LANES>(rho_dissipation);
-#pragma unroll
-        for (int d = 0; d < D; ++d)
-            force[d] = fx::group_sum<LANES>(force[d]);
-    }
+    if (general)
+        sums.get(force, &rho_dissipation);
     else
     {
-        fixed_1st<D, LANES>(n, i, sub, in, fp.value, force, &rho_dissipation);
+        value_1st<D>(sums, force, &rho_dissipation);
         const double scale = in.factor * p0 * f.Vol[0];
         rho_dissipation *= scale;
 #pragma unroll
         for (int d = 0; d < D; ++d)
             force[d] *= scale;
     }
-    if (wn.count && LANES == 1)
-    {
-        if (wn.count[i] > 0)
-        {
-#pragma unroll
-            for (int d = 0; d < D; ++d)
-                force[d] += wall_sum[d * n + i];
-            rho_dissipation += wall_sum[D * n + i];
-        }
-    }
-    else if (wn.count)
-    {
-        double wf[3] = {0, 0, 0}, wr = 0;
-        wall_1st<D, LANES>(n, i, sub, f, wn, w, wf, &wr);
-        rho_dissipation += fx::group_sum<LANES>(wr);
-#pragma unroll
-        for (int d = 0; d < D; ++d)
-            force[d] += fx::group_sum<LANES>(wf[d]);
-    }
-    if (sub != 0)
-        return;
+    add_walls<D, LANES>(n, i, wn, sums, wall_sum, force, &rho_dissipation);
     const double Vol_i = f.Vol[i], dt_m = dt / f.mass[i];
     f.drho_dt[i] = rho_dissipation * rs.inv_rho0c0_ave * f.rho[i];
 #pragma unroll
@@ -691,52 +808,52 @@ __global__ void __launch_bounds__(kBlock, kBlocks2)
                    const double *__restrict__ wall_sum)
 {
     const size_t g = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    const size_t i = g / LANES;
+    size_t i = g / LANES;
     const unsigned sub = unsigned(g % LANES);
-    if (i >= n)
-        return;
     // the jump rho0c0_geo_ave u min(beta max(u, 0), 1): the constants are applied to the sums
     const double beta = rs.slope * rs.inv_c0_ave;
+    const bool general = !fv.value || __ldcg(fv.flag) == fv.epoch;
+    SweepSums<D> sums;
+    if (i < n)
+    {
+        if (general)
+        {
+            double diss[3] = {0, 0, 0}, rate = 0;
+            general_2nd<D>(n, i, sub, LANES, f.vel, f.Vol, in, beta, diss, &rate);
+            rate = fx::group_sum<LANES>(rate);
+#pragma unroll
+            for (int d = 0; d < D; ++d)
+                diss[d] = fx::group_sum<LANES>(diss[d]);
+            sums.set(diss, rate);
+        }
+        else
+            fixed_2nd<D, LANES>(n, i, sub, in, fv.value, velocity_unit(fv), 1.0 / beta, sums);
+        if (walls_in_sweep<D, LANES>() && wn.count)
+        {
+            double wf[3] = {0, 0, 0}, wr = 0;
+            wall_2nd<D, LANES>(n, i, sub, f, wn, w, beta, wf, &wr);
+            sums.wall[D] = fx::group_sum<LANES>(wr);
+#pragma unroll
+            for (int d = 0; d < D; ++d)
+                sums.wall[d] = fx::group_sum<LANES>(wf[d]);
+        }
+    }
+    if (!pack_particles<D, LANES>(n, sub, i, sums))
+        return;
     double diss[3] = {0, 0, 0};
     double rate = 0;
-    if (!fv.value || __ldcg(fv.flag) == fv.epoch)
-    {
-        general_2nd<D>(n, i, sub, LANES, f.vel, f.Vol, in, beta, diss, &rate);
-        rate = fx::group_sum<LANES>(rate);
-#pragma unroll
-        for (int d = 0; d < D; ++d)
-            diss[d] = fx::group_sum<LANES>(diss[d]);
-    }
+    if (general)
+        sums.get(diss, &rate);
     else
     {
-        fixed_2nd<D, LANES>(n, i, sub, in, fv.value, velocity_unit(fv), 1.0 / beta, diss, &rate);
+        value_2nd<D>(sums, velocity_unit(fv), diss, &rate);
         const double scale = in.factor * f.Vol[0];
         rate *= scale;
 #pragma unroll
         for (int d = 0; d < D; ++d)
             diss[d] *= scale * beta;
     }
-    if (wn.count && LANES == 1)
-    {
-        if (wn.count[i] > 0)
-        {
-#pragma unroll
-            for (int d = 0; d < D; ++d)
-                diss[d] += wall_sum[d * n + i];
-            rate += wall_sum[D * n + i];
-        }
-    }
-    else if (wn.count)
-    {
-        double wf[3] = {0, 0, 0}, wr = 0;
-        wall_2nd<D, LANES>(n, i, sub, f, wn, w, beta, wf, &wr);
-        rate += fx::group_sum<LANES>(wr);
-#pragma unroll
-        for (int d = 0; d < D; ++d)
-            diss[d] += fx::group_sum<LANES>(wf[d]);
-    }
-    if (sub != 0)
-        return;
+    add_walls<D, LANES>(n, i, wn, sums, wall_sum, diss, &rate);
     const double rho_i = f.rho[i], Vol_i = f.Vol[i];
     const double drho = f.drho_dt[i] + rate * rho_i;
     f.drho_dt[i] = drho;
@@ -1062,16 +1179,19 @@ Fixed fixed_path(Fixed f, const InnerPairs &in, double beta = 0.0)
     return f;
 }
 
-// Threads per particle of the sweeps; the sums do not depend on it.
+// Threads per particle of the sweeps; the sums do not depend on it.  Below 512 threads per SM
+// a particle is shared by up to 8 threads (4 in 2D, whose lists hold about 20 entries): 3D,
+// 90,000 particles 2,500 us a step with 2 threads each (1,024 per SM), 1,940 with one; 46,000
+// particles 1,362 with two, 1,465 with one.
 int sweep_lanes(sphx_ctx ctx, int dim, size_t n)
 {
-    const size_t want = size_t(std::max(1, ctx->num_sms)) * 1024;
+    const size_t want = size_t(std::max(1, ctx->num_sms)) * 512;
     int lanes = 1;
     while (lanes < (dim == 2 ? 4 : 8) && n * lanes < want)
         lanes *= 2;
     return lanes;
 }
-// The wall terms of a sweep that takes them from the relation's workspace (see k_wall).
+// The wall terms of a sweep, into the relation's workspace (see k_wall).
 template <int HALF>
 int wall_terms(sphx_relation wall, const FluidVars &f, const Neighbors &wn, const WallVars &w, double beta)
 {
@@ -1080,7 +1200,8 @@ int wall_terms(sphx_relation wall, const FluidVars &f, const Neighbors &wn, cons
     sphx_ctx ctx = wall->ctx;
     const int dim = wall->src->dim;
     const size_t n = wall->src->n, na = wall->n_active;
-    if (sweep_lanes(ctx, dim, n) > 1)
+    const int lanes = sweep_lanes(ctx, dim, n);
+    if (lanes == (dim == 2 ? 4 : 8)) // walls_in_sweep
         return SPHX_OK;
     const unsigned grid = grid_for(na * kWallLanes, kBlock);
     if (dim == 2)

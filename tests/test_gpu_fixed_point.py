@@ -17,8 +17,8 @@ pytestmark = pytest.mark.gpu
 TOL = 3e-11
 
 # threads per particle: 4, 2, 1 in 2D; 8, 4, 2, 1 in 3D
-SIZES = {"2d-4": (2, 0.025), "2d-2": (2, 0.005), "2d-1": (2, 0.0035), "3d-8": (3, 0.06), "3d-4": (3, 0.026),
-         "3d-2": (3, 0.02), "3d-1": (3, 0.0165)}
+SIZES = {"2d-4": (2, 0.025), "2d-2": (2, 0.0055), "2d-1": (2, 0.0045), "3d-8": (3, 0.06), "3d-4": (3, 0.03),
+         "3d-2": (3, 0.025), "3d-1": (3, 0.02)}
 
 
 def state(case, n, speed, compression, spread, seed):
