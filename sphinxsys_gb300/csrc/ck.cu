@@ -23,17 +23,20 @@
 // update): each fused update touches only the particle's own variables, which no other
 // particle reads in that interaction.
 //
-// Bound: the FP64 pipe (2 lanes a cycle per SM on GB300), so the sweeps are written for few
-// FP64 instructions a pair: one reciprocal square root for distance and direction, the table
-// as polynomial coefficients (3 fused multiply-adds; its Lagrange form takes 5 divisions),
-// factors common to a particle's pairs applied to the sums.  One advection step of the 3D
-// dam break at dp = 0.02 (90,000 particles): 34.8 -> 10.6 ms, error against 64-bit
-// references 2.2e-13 -> 1.9e-13.
+// Bound: the FP64 pipe (2 lanes a cycle per SM on GB300), so the once-per-step sums are
+// written for few FP64 instructions a pair: one reciprocal square root for distance and
+// direction, the table as polynomial coefficients (3 fused multiply-adds; its Lagrange form
+// takes 5 divisions), factors common to a particle's pairs applied to the sums.  The half
+// steps keep the pair geometry between relation updates and sum in fixed point.  One
+// advection step of the 3D dam break at dp = 0.02 (90,000 particles): 35.2 ms, 10.0 with the
+// lighter FP64 sums, 4.7 with the fixed-point half steps (a 1st / 2nd half 0.70 / 0.87 ->
+// 0.13 / 0.18 ms); error against 64-bit references 2.2e-13, 1.9e-13, 1.9e-13.
 #include <algorithm>
 #include <cmath>
 #include <string>
 #include <vector>
 
+#include "fx.cuh"
 #include "sphx_device.cuh"
 #include "sphx_internal.cuh"
 
@@ -229,6 +232,21 @@ __device__ __forceinline__ void matvec(const double *B, size_t n, size_t i, cons
 #pragma unroll
         for (int b = 1; b < D; ++b)
             s = fma(B[(a * D + b) * n + i], x[b], s);
+        y[a] = s;
+    }
+}
+
+// y = B x for a matrix in registers
+template <int D>
+__device__ __forceinline__ void corrected(const double *B, const double *x, double *y)
+{
+#pragma unroll
+    for (int a = 0; a < D; ++a)
+    {
+        double s = B[a * D] * x[0];
+#pragma unroll
+        for (int b = 1; b < D; ++b)
+            s = fma(B[a * D + b], x[b], s);
         y[a] = s;
     }
 }
@@ -453,8 +471,85 @@ __global__ void __launch_bounds__(kBlock)
         }
 }
 
+// ---------------------------------------------------------------- acoustic half steps
+// The pair geometry does not change between relation updates while the particles stay where
+// they were, so the tabulated kernel derivative and the unit vector of every pair are formed
+// once per list (k_ck_pairs) and the inner sums of the half steps run in fixed point on them
+// (fx.cuh).  The kernels that convert the particle values compare the positions with those
+// the pairs were made from; if one moved, or a value lies outside the format (|p| >= p0 / 4,
+// |B| >= 4, a volume four times the first particle's), the sweeps take their general path,
+// FP64 from the current positions.
+constexpr int kMatrixBits = 58; // correction matrix
+
+// Particle record of the 1st half: pressure, volume, matrix; of the 2nd: velocity, volume.
 template <int D>
-__global__ void k_ck_init1(size_t n, CKFluid f, CKParams k, double dt)
+struct Rec1
+{
+    static constexpr int words = 2 + D * D + (D == 3 ? 1 : 0); // 12 or 6, whole 16-byte pairs
+};
+
+struct CKPairs
+{
+    const uint32_t *count, *J;
+    fx::EntryStore at;
+    unsigned cap;
+    uint32_t limit;
+    double factor; // of the tabulated derivative
+    const double *pos; // positions the entries were made from
+    bool general;      // lists or parameters the integer sums cannot take
+};
+
+template <int D, int LANES>
+__global__ void __launch_bounds__(kBlock) k_ck_pairs(size_t n, const double *__restrict__ pos, Lists in, TabK t,
+                                                     double inv_factor, fx::EntryStore at, double *__restrict__ copy)
+{
+    __shared__ double rows[kIntervals * kRow];
+    load_rows(rows, t.dw);
+    const Group<LANES> g;
+    const size_t i = g.i;
+    if (i >= n)
+        return;
+    double x_i[3], r[3], inv;
+    load_point<D>(pos, n, i, x_i);
+    const unsigned c = min(in.count[i], in.cap);
+    for (unsigned s = g.sub; s < c; s += LANES)
+    {
+        const size_t slot = size_t(s) * n + i;
+        const uint32_t j = in.J[slot];
+        if (!entry_ok(in, j))
+            continue;
+        const double n2 = separation<D>(x_i, pos, n, j, r, inv);
+        fx::Entry<D> q;
+        q.k = fx::encode(tabulated(rows, (n2 * inv) * t.inv_step) * inv_factor);
+#pragma unroll
+        for (int a = 0; a < D; ++a)
+            q.e[a] = fx::encode(r[a] * inv);
+        at.store<D>(slot, q);
+    }
+    if (g.leads())
+#pragma unroll
+        for (int a = 0; a < D; ++a)
+            copy[a * n + i] = x_i[a];
+}
+
+template <int D>
+__device__ __forceinline__ bool stayed(const double *pos, const double *copy, size_t n, size_t i)
+{
+    bool same = true;
+#pragma unroll
+    for (int a = 0; a < D; ++a)
+        same = same && __double_as_longlong(pos[a * n + i]) == __double_as_longlong(copy[a * n + i]);
+    return same;
+}
+
+// The unit of the volumes: 57 bits hold up to four times the first particle's.
+__device__ __forceinline__ int volume_unit(const double *Vol)
+{
+    return ((__double2hiint(Vol[0]) >> 20) & 0x7ff) - 1022 + 2 - fx::kListBits;
+}
+
+template <int D>
+__global__ void k_ck_init1(size_t n, CKFluid f, CKParams k, double dt, CKPairs pr, fx::Fixed fp)
 {
     size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
     if (i >= n)
@@ -463,47 +558,317 @@ __global__ void k_ck_init1(size_t n, CKFluid f, CKParams k, double dt)
     f.compression[i] = comp;
     double rho = comp * k.rho0;
     f.rho[i] = rho;
-    f.p[i] = k.p0 * (rho / k.rho0 - 1.0);
+    const double x = rho / k.rho0 - 1.0;
+    f.p[i] = k.p0 * x;
+#pragma unroll
     for (int a = 0; a < D; ++a)
         f.dpos[a * n + i] += f.vel[a * n + i] * dt * 0.5;
+    bool fits = fabs(x) < fx::kPressureRange && stayed<D>(f.pos, pr.pos, n, i);
+    long long *out = fp.value + i * Rec1<D>::words;
+    out[0] = fits ? __double2ll_rn(x * fx::pow2(fx::kPressureBits)) : 0;
+    const long long v = fx::fixed(f.Vol[i], volume_unit(f.Vol), fits);
+    fits = fits && v >= 0 && v < (1ll << fx::kListBits) && abs(volume_unit(f.Vol)) < 250;
+    out[1] = v;
+#pragma unroll
+    for (int q = 0; q < D * D; ++q)
+        out[2 + q] = fx::fixed(f.B[q * n + i], -kMatrixBits, fits);
+    if (!fits)
+        *fp.flag = fp.epoch;
 }
 
-// AverageP of both corrections: sum_j (p_i B_j + p_j B_i) e dW V_j =
-// p_i sum_j (B_j e) dW V_j + B_i sum_j p_j e dW V_j, so the pair needs one matrix product.
-template <int D, int LANES>
-__global__ void __launch_bounds__(kBlock) k_ck_interact1(size_t n, CKFluid f, CKWall w, Lists in, Lists wl, TabK t,
-                                                         CKParams k, double dt)
+// Velocities (units of velocity_unit) and volumes: records of four words.
+template <int D>
+__global__ void k_ck_init2(size_t n, CKFluid f, CKPairs pr, fx::Fixed fv)
 {
-    __shared__ double rows[kIntervals * kRow];
-    load_rows(rows, t.dw);
-    const Group<LANES> g;
-    const size_t i = g.i;
+    size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
     if (i >= n)
         return;
-    const double p_i = f.p[i];
-    double x_i[3], r[3], e[3], bj[3], inv;
-    load_point<D>(f.pos, n, i, x_i);
-    double fj[3] = {0, 0, 0}, fi[3] = {0, 0, 0}, dis = 0;
-    for_each_neighbor(in, g, [&](uint32_t j) {
-        const double n2 = separation<D>(x_i, f.pos, n, j, r, inv);
-        const double dWV = tabulated(rows, (n2 * inv) * t.inv_step) * f.Vol[j];
-        const double p_j = f.p[j], kj = p_j * dWV;
+    const int unit = fx::velocity_unit(fv);
+    bool fits = unit < 200 && stayed<D>(f.pos, pr.pos, n, i);
+    long long q[4] = {0, 0, 0, 0};
 #pragma unroll
-        for (int a = 0; a < D; ++a)
-            e[a] = r[a] * inv;
-        matvec<D>(f.B, n, j, e, bj);
+    for (int d = 0; d < D; ++d)
+        q[d] = fx::fixed(f.vel[d * n + i], unit, fits);
+    q[3] = fx::fixed(f.Vol[i], volume_unit(f.Vol), fits);
+    fits = fits && q[3] >= 0 && q[3] < (1ll << fx::kListBits) && abs(volume_unit(f.Vol)) < 250;
+#pragma unroll
+    for (int d = 0; d < D * D; ++d) // the particle's own matrix is converted in the sweep
+    {
+        const double b = f.B[d * n + i];
+        fits = fits && fabs(b) < 4.0;
+    }
+    longlong2 *out = reinterpret_cast<longlong2 *>(fv.value) + 2 * i;
+    out[0] = make_longlong2(q[0], q[1]);
+    out[1] = make_longlong2(q[2], q[3]);
+    if (!fits)
+        *fv.flag = fv.epoch;
+}
+
+// K V_j in list-entry form, in the unit of the volumes.
+__device__ __forceinline__ int2 weighted(int2 K, long long V)
+{
+    const fx::Halves k{K.x, K.y}, v = fx::halves(V);
+    return fx::split((fx::mad(k.h, v.h, 0) << 5) + (fx::middle(k, v, 1 << 25) >> 26));
+}
+
+// A 64-bit factor times a list entry: hh 2^63 + m 2^32.
+__device__ __forceinline__ void times(long long v, int2 e, long long &hh, long long &m)
+{
+    const int vh = fx::high(v), vl = fx::low(v);
+    hh = fx::mad(vh, e.x, hh);
+    m = fx::mad(vh, e.y, m);
+    m = fx::mad(vl, e.x, m);
+    m = fx::low_product(vl, e.y, m);
+}
+
+// The pairs of this thread's share of particle i: f(entry, j), the entry of the next pair
+// loaded while this one is computed.
+template <int D, int LANES, class F>
+__device__ __forceinline__ void for_pairs(const CKPairs &in, size_t n, const Group<LANES> &g, F &&f)
+{
+    const unsigned cnt = min(in.count[g.i], in.cap);
+    size_t slot = size_t(g.sub) * n + g.i;
+    const size_t step = size_t(LANES) * n;
+    fx::Entry<D> next{};
+    uint32_t jn = uint32_t(g.i);
+    if (g.sub < cnt)
+    {
+        jn = in.J[slot];
+        next = in.at.load<D>(slot);
+    }
+    for (unsigned s = g.sub; s < cnt; s += LANES)
+    {
+        const fx::Entry<D> q = next;
+        const uint32_t j = jn;
+        slot += step;
+        if (s + LANES < cnt)
+        {
+            jn = in.J[slot];
+            next = in.at.load<D>(slot);
+        }
+        if (SPHX_CHECKED(j < in.limit, kCheckListEntry, j))
+            f(q, j);
+    }
+}
+
+// The inner sums of the 1st half: fj = sum (B_j e) dW V_j, fi = sum p_j e dW V_j,
+// dis = sum (p_i - p_j) dW V_j, over the prefactor of dW and (fi, dis) p0.
+template <int D, int LANES>
+__device__ __forceinline__ void ck_fixed_1st(size_t n, const Group<LANES> &g, const CKPairs &in, const fx::Fixed &fp,
+                                             int vu, double *fj, double *fi, double *dis)
+{
+    constexpr int W = Rec1<D>::words;
+    const long long P_i = fp.value[g.i * W];
+    fx::Sum A[D], F[D], S;
+    fx::Align ab, ap;
+    int folded = 0;
+    bool first = true;
+    for_pairs<D>(in, n, g, [&](const fx::Entry<D> &q, uint32_t j) {
+        long long rec[W];
+        const longlong2 *src = reinterpret_cast<const longlong2 *>(fp.value + size_t(j) * W);
+#pragma unroll
+        for (int w = 0; w < W / 2; ++w)
+        {
+            const longlong2 v = __ldg(src + w);
+            rec[2 * w] = v.x;
+            rec[2 * w + 1] = v.y;
+        }
+        const int2 KV = weighted(q.k, rec[1]);
+        S.add(fx::high(P_i - rec[0]), fx::low(P_i - rec[0]), KV);
+        long long hp = 0, mp = 0, hh[D], m[D];
+        times(rec[0], KV, hp, mp);
+        int tb = 0, tp = 0;
+        fx::Align::see(tp, hp);
 #pragma unroll
         for (int a = 0; a < D; ++a)
         {
-            fj[a] = fma(dWV, bj[a], fj[a]);
-            fi[a] = fma(kj, e[a], fi[a]);
+            hh[a] = m[a] = 0;
+#pragma unroll
+            for (int b = 0; b < D; ++b)
+                times(rec[2 + a * D + b], q.e[b], hh[a], m[a]);
+            fx::Align::see(tb, hh[a]);
         }
-        dis = fma(p_i - p_j, dWV, dis);
+        if (first)
+        {
+            first = false;
+            ab.start(tb);
+            ap.start(tp);
+        }
+        while (ab.over(tb))
+        {
+            const int k = ab.step();
+#pragma unroll
+            for (int a = 0; a < D; ++a)
+                A[a].shift(k);
+        }
+        while (ap.over(tp))
+        {
+            const int k = ap.step();
+#pragma unroll
+            for (int a = 0; a < D; ++a)
+                F[a].shift(k);
+        }
+        const long long T = ap.apply(hp, mp);
+        const int th = int(T >> 31), tl = int(unsigned(T) & 0x7fffffffu);
+#pragma unroll
+        for (int a = 0; a < D; ++a)
+        {
+            F[a].add(th, tl, q.e[a]);
+            const long long U = ab.apply(hh[a], m[a]);
+            A[a].add(int(U >> 31), int(unsigned(U) & 0x7fffffffu), KV);
+        }
+        if (++folded == fx::kFold)
+        {
+            folded = 0;
+            S.fold();
+#pragma unroll
+            for (int a = 0; a < D; ++a)
+            {
+                F[a].fold();
+                A[a].fold();
+            }
+        }
     });
-    double wf[3] = {0, 0, 0}, wdis = 0;
-    if (wl.J)
+    const int ga = fx::group_min<LANES>(first ? fx::Align::kMost : ab.a);
+    const int gp = fx::group_min<LANES>(first ? fx::Align::kMost : ap.a);
+    fx::group_sum<LANES>(S);
+    *dis = S.value() * fx::pow2(32 - fx::kPressureBits + vu);
+#pragma unroll
+    for (int a = 0; a < D; ++a)
     {
-        const double rho_i = f.rho[i], inv_m = 1.0 / f.mass[i];
+        if (LANES > 1 && !first)
+        {
+            A[a].shift(ab.a - ga);
+            F[a].shift(ap.a - gp);
+        }
+        fx::group_sum<LANES>(A[a]);
+        fx::group_sum<LANES>(F[a]);
+        fj[a] = A[a].value() * fx::pow2(94 - ga - kMatrixBits - fx::kListBits + vu);
+        fi[a] = F[a].value() * fx::pow2(94 - gp - fx::kPressureBits - fx::kListBits + vu);
+    }
+}
+
+// The inner sums of the 2nd half, u = (v_i - v_j) . e: div = sum (v_i - v_j) . (B_i e) dW V_j and
+// pd = sum u min(u+, u_lim) dW V_j e, over the prefactor of dW.
+template <int D, int LANES>
+__device__ __forceinline__ void ck_fixed_2nd(size_t n, const Group<LANES> &g, const CKPairs &in, const fx::Fixed &fv,
+                                             int vu, const double *B, double u_lim, double *pd, double *div)
+{
+    const int unit = fx::velocity_unit(fv);
+    long long v_i[3], Bi[D * D];
+    {
+        const longlong2 *own = reinterpret_cast<const longlong2 *>(fv.value) + 2 * g.i;
+        const longlong2 x = own[0], y = own[1];
+        v_i[0] = x.x;
+        v_i[1] = x.y;
+        v_i[2] = y.x;
+    }
+    bool fits = true;
+#pragma unroll
+    for (int q = 0; q < D * D; ++q)
+        Bi[q] = fx::fixed(B[q], -kMatrixBits, fits);
+    fx::Sum F[D], S;
+    fx::Align aw, au;
+    // u at alignment 0 is in units of 2^(63 - kListBits + unit)
+    const double l = u_lim * fx::pow2(fx::kListBits - 63 - unit);
+    const long long t_lim = l < 1.0e17 ? __double2ll_rn(l) : 1ll << 57;
+    long long lim = 0;
+    int folded = 0;
+    bool first = true;
+    for_pairs<D>(in, n, g, [&](const fx::Entry<D> &q, uint32_t j) {
+        const longlong2 *src = reinterpret_cast<const longlong2 *>(fv.value) + 2 * size_t(j);
+        const longlong2 x = __ldg(src), y = __ldg(src + 1);
+        const long long dv[3] = {v_i[0] - x.x, v_i[1] - x.y, v_i[2] - y.x};
+        const int2 KV = weighted(q.k, y.y);
+        long long hu = 0, mu = 0, hw = 0, mw = 0;
+#pragma unroll
+        for (int a = 0; a < D; ++a)
+        {
+            long long hb = 0, mb = 1 << 28; // B_i e in units of 2^-54, rounded
+#pragma unroll
+            for (int b = 0; b < D; ++b)
+                times(Bi[a * D + b], q.e[b], hb, mb);
+            times(dv[a], fx::split((hb << 2) + (mb >> 29)), hw, mw);
+            times(dv[a], q.e[a], hu, mu);
+        }
+        int tu = 0, tw = 0;
+        fx::Align::see(tu, hu);
+        fx::Align::see(tw, hw);
+        if (first)
+        {
+            first = false;
+            au.start(tu);
+            aw.start(tw);
+            lim = fx::limit_at(t_lim, au.a);
+        }
+        while (aw.over(tw))
+            S.shift(aw.step());
+        while (au.over(tu))
+        {
+            const int k = au.step();
+            lim = fx::limit_at(t_lim, au.a);
+#pragma unroll
+            for (int a = 0; a < D; ++a)
+                F[a].shift(2 * k);
+        }
+        const long long w = aw.apply(hw, mw);
+        S.add(int(w >> 31), int(unsigned(w) & 0x7fffffffu), KV);
+        long long sc[1];
+        fx::jump(au.apply(hu, mu), KV, lim, nullptr, sc);
+        const int sh = int(sc[0] >> 31), sl = int(unsigned(sc[0]) & 0x7fffffffu);
+#pragma unroll
+        for (int a = 0; a < D; ++a)
+            F[a].add(sh, sl, q.e[a]);
+        if (++folded == fx::kFold)
+        {
+            folded = 0;
+            S.fold();
+#pragma unroll
+            for (int a = 0; a < D; ++a)
+                F[a].fold();
+        }
+    });
+    const int gw = fx::group_min<LANES>(first ? fx::Align::kMost : aw.a);
+    const int gu = fx::group_min<LANES>(first ? fx::Align::kMost : au.a);
+    if (LANES > 1 && !first)
+        S.shift(aw.a - gw);
+    fx::group_sum<LANES>(S);
+    *div = S.value() * fx::pow2(40 - gw + unit + vu);
+#pragma unroll
+    for (int a = 0; a < D; ++a)
+    {
+        if (LANES > 1 && !first)
+        {
+            F[a].shift(au.a - gu);
+            F[a].shift(au.a - gu);
+        }
+        fx::group_sum<LANES>(F[a]);
+        pd[a] = F[a].value() * fx::pow2(96 - 2 * gu + 2 * unit + vu);
+    }
+}
+
+// The wall terms of the particles that have wall neighbours, kWallLanes threads each, into
+// sum[c n + i]: the 1st half's force before the matrix B_i and its dissipation, the 2nd half's
+// dissipation force over rho0c0_geo_ave and its divergence.  A warp of the inner sweeps would run
+// as many wall pairs as its longest wall list, on the FP64 pipe.
+constexpr int kWallLanes = 16; // one step, 8,000 particles: 1,354 us with 4 threads, 1,195 with 8, 1,164 with 16, 1,644 with 2
+template <int D, int HALF>
+__global__ void __launch_bounds__(kBlock) k_ck_wall(size_t n, size_t n_active, const uint32_t *__restrict__ active,
+                                                    CKFluid f, CKWall w, Lists wl, TabK t, CKParams k,
+                                                    double *__restrict__ sum)
+{
+    __shared__ double rows[kIntervals * kRow];
+    load_rows(rows, t.dw);
+    Group<kWallLanes> g;
+    if (g.i >= n_active)
+        return;
+    g.i = active[g.i];
+    const size_t i = g.i;
+    double x_i[3], r[3], e[3], inv, out[3] = {0, 0, 0}, q = 0;
+    load_point<D>(f.pos, n, i, x_i);
+    if (HALF == 1)
+    {
+        const double p_i = f.p[i], rho_i = f.rho[i], inv_m = 1.0 / f.mass[i];
         double acc_i[3];
 #pragma unroll
         for (int a = 0; a < D; ++a)
@@ -523,94 +888,21 @@ __global__ void __launch_bounds__(kBlock) k_ck_interact1(size_t n, CKFluid f, CK
             const double sc = (p_i + p_wall) * dWV;
 #pragma unroll
             for (int a = 0; a < D; ++a)
-                wf[a] = fma(sc, e[a], wf[a]);
-            wdis = fma(p_i - p_wall, dWV, wdis);
+                out[a] = fma(sc, e[a], out[a]);
+            q = fma(p_i - p_wall, dWV, q);
         });
     }
-    dis = g.sum(dis);
-#pragma unroll
-    for (int a = 0; a < D; ++a)
+    else
     {
-        fj[a] = g.sum(fj[a]);
-        fi[a] = g.sum(fi[a]);
-    }
-    if (wl.J)
-    {
-        wdis = g.sum(wdis);
+        double v_i[3], B[D * D], du[3], be[3], nj[3];
+        load_point<D>(f.vel, n, i, v_i);
 #pragma unroll
-        for (int a = 0; a < D; ++a)
-            wf[a] = g.sum(wf[a]);
-    }
-    if (!g.leads())
-        return;
-    double be[3];
-#pragma unroll
-    for (int a = 0; a < D; ++a)
-        fi[a] = 2.0 * k.inv_Zsum * k.Z * fi[a] + wf[a];
-    matvec<D>(f.B, n, i, fi, be);
-    const double Vol_i = f.Vol[i], m_i = f.mass[i], pz = 2.0 * k.inv_Zsum * k.Z * p_i;
-    f.rate[i] = (dis + wdis) * k.inv_rho0c0_ave * f.compression[i];
-#pragma unroll
-    for (int a = 0; a < D; ++a)
-    {
-        const double F = f.force[a * n + i] - (pz * fj[a] + be[a]) * Vol_i;
-        f.force[a * n + i] = F;
-        f.vel[a * n + i] += (f.force_prior[a * n + i] + F) / m_i * dt;
-    }
-}
-
-// AverageV: 2 (v_i - v_ave) = v_i - v_j, so the divergence is sum_j (v_i - v_j) . (B_i e) dW V_j.
-template <int D, int LANES>
-__global__ void __launch_bounds__(kBlock) k_ck_second(size_t n, CKFluid f, CKWall w, Lists in, Lists wl, TabK t,
-                                                      CKParams k, double dt)
-{
-    __shared__ double rows[kIntervals * kRow];
-    load_rows(rows, t.dw);
-    const Group<LANES> g;
-    const size_t i = g.i;
-    if (i >= n)
-        return;
-    double v_i[3] = {0, 0, 0}, x_i[3], B[D * D];
-    load_point<D>(f.vel, n, i, v_i);
-    load_point<D>(f.pos, n, i, x_i);
-#pragma unroll
-    for (int a = 0; a < D * D; ++a)
-        B[a] = f.B[a * n + i];
-    const double beta = k.slope * k.inv_c0_ave;
-    double div = 0, pd[3] = {0, 0, 0};
-    double r[3], e[3], du[3], be[3], inv;
-    auto corrected = [&]() {
-#pragma unroll
-        for (int a = 0; a < D; ++a)
-        {
-            double s = B[a * D] * e[0];
-#pragma unroll
-            for (int b = 1; b < D; ++b)
-                s = fma(B[a * D + b], e[b], s);
-            be[a] = s;
-        }
-    };
-    for_each_neighbor(in, g, [&](uint32_t j) {
-        const double n2 = separation<D>(x_i, f.pos, n, j, r, inv);
-        const double dWV = tabulated(rows, (n2 * inv) * t.inv_step) * f.Vol[j];
-#pragma unroll
-        for (int a = 0; a < D; ++a)
-        {
-            e[a] = r[a] * inv;
-            du[a] = v_i[a] - f.vel[a * n + j];
-        }
-        corrected();
-        div = fma(dot<D>(du, be), dWV, div);
-        const double pj = limited_jump(beta, dot<D>(du, e), dWV);
-#pragma unroll
-        for (int a = 0; a < D; ++a)
-            pd[a] = fma(pj, e[a], pd[a]);
-    });
-    if (wl.J)
+        for (int a = 0; a < D * D; ++a)
+            B[a] = f.B[a * n + i];
+        const double beta = k.slope * k.inv_c0_ave;
         for_each_neighbor(wl, g, [&](uint32_t j) {
             const double n2 = separation<D>(x_i, w.pos, w.nw, j, r, inv);
             const double dWV = tabulated(rows, (n2 * inv) * t.inv_step) * w.Vol[j];
-            double nj[3];
 #pragma unroll
             for (int a = 0; a < D; ++a)
             {
@@ -618,21 +910,167 @@ __global__ void __launch_bounds__(kBlock) k_ck_second(size_t n, CKFluid f, CKWal
                 du[a] = 2.0 * (v_i[a] - w.vel_ave[a * w.nw + j]);
                 nj[a] = w.n[a * w.nw + j];
             }
-            corrected();
-            div = fma(dot<D>(du, be), dWV, div);
+            corrected<D>(B, e, be);
+            q = fma(dot<D>(du, be), dWV, q);
             const double en = dot<D>(e, nj);
             const double sgn = en > 0 ? 1.0 : (en < 0 ? -1.0 : 0.0);
             const double pj = limited_jump(beta, sgn * dot<D>(du, nj), dWV) * sgn;
 #pragma unroll
             for (int a = 0; a < D; ++a)
-                pd[a] = fma(pj, nj[a], pd[a]);
+                out[a] = fma(pj, nj[a], out[a]);
         });
-    div = g.sum(div);
+    }
+    q = g.sum(q);
 #pragma unroll
     for (int a = 0; a < D; ++a)
-        pd[a] = g.sum(pd[a]);
+        out[a] = g.sum(out[a]);
     if (!g.leads())
         return;
+#pragma unroll
+    for (int a = 0; a < D; ++a)
+        sum[a * n + i] = out[a];
+    sum[D * n + i] = q;
+}
+
+// AverageP of both corrections: sum_j (p_i B_j + p_j B_i) e dW V_j =
+// p_i sum_j (B_j e) dW V_j + B_i sum_j p_j e dW V_j, so the pair needs one matrix product.
+template <int D, int LANES>
+__global__ void __launch_bounds__(kBlock, 4)
+    k_ck_interact1(size_t n, CKFluid f, Lists in, CKPairs pr, fx::Fixed fp, TabK t, CKParams k, double dt,
+                   const uint32_t *__restrict__ wall_count, const double *__restrict__ wall_sum)
+{
+    __shared__ double rows[kIntervals * kRow];
+    const bool general = pr.general || __ldcg(fp.flag) == fp.epoch;
+    if (general)
+        load_rows(rows, t.dw);
+    const Group<LANES> g;
+    const size_t i = g.i;
+    if (i >= n)
+        return;
+    const double p_i = f.p[i];
+    double fj[3] = {0, 0, 0}, fi[3] = {0, 0, 0}, dis = 0;
+    if (general)
+    {
+        double x_i[3], r[3], e[3], bj[3], inv;
+        load_point<D>(f.pos, n, i, x_i);
+        for_each_neighbor(in, g, [&](uint32_t j) {
+            const double n2 = separation<D>(x_i, f.pos, n, j, r, inv);
+            const double dWV = tabulated(rows, (n2 * inv) * t.inv_step) * f.Vol[j];
+            const double p_j = f.p[j], kj = p_j * dWV;
+#pragma unroll
+            for (int a = 0; a < D; ++a)
+                e[a] = r[a] * inv;
+            matvec<D>(f.B, n, j, e, bj);
+#pragma unroll
+            for (int a = 0; a < D; ++a)
+            {
+                fj[a] = fma(dWV, bj[a], fj[a]);
+                fi[a] = fma(kj, e[a], fi[a]);
+            }
+            dis = fma(p_i - p_j, dWV, dis);
+        });
+        dis = g.sum(dis);
+#pragma unroll
+        for (int a = 0; a < D; ++a)
+        {
+            fj[a] = g.sum(fj[a]);
+            fi[a] = g.sum(fi[a]);
+        }
+    }
+    else
+    {
+        ck_fixed_1st<D, LANES>(n, g, pr, fp, volume_unit(f.Vol), fj, fi, &dis);
+        const double s = pr.factor * k.p0;
+        dis *= s;
+#pragma unroll
+        for (int a = 0; a < D; ++a)
+        {
+            fj[a] *= pr.factor;
+            fi[a] *= s;
+        }
+    }
+    if (!g.leads())
+        return;
+    double be[3];
+    const bool wall = wall_count && wall_count[i] > 0;
+#pragma unroll
+    for (int a = 0; a < D; ++a)
+        fi[a] = 2.0 * k.inv_Zsum * k.Z * fi[a] + (wall ? wall_sum[a * n + i] : 0.0);
+    matvec<D>(f.B, n, i, fi, be);
+    const double Vol_i = f.Vol[i], dt_m = dt / f.mass[i], pz = 2.0 * k.inv_Zsum * k.Z * p_i;
+    f.rate[i] = (dis + (wall ? wall_sum[D * n + i] : 0.0)) * k.inv_rho0c0_ave * f.compression[i];
+#pragma unroll
+    for (int a = 0; a < D; ++a)
+    {
+        const double F = f.force[a * n + i] - (pz * fj[a] + be[a]) * Vol_i;
+        f.force[a * n + i] = F;
+        f.vel[a * n + i] += (f.force_prior[a * n + i] + F) * dt_m;
+    }
+}
+
+// AverageV: 2 (v_i - v_ave) = v_i - v_j, so the divergence is sum_j (v_i - v_j) . (B_i e) dW V_j.
+template <int D, int LANES>
+__global__ void __launch_bounds__(kBlock, 4)
+    k_ck_second(size_t n, CKFluid f, Lists in, CKPairs pr, fx::Fixed fv, TabK t, CKParams k, double dt,
+                const uint32_t *__restrict__ wall_count, const double *__restrict__ wall_sum)
+{
+    __shared__ double rows[kIntervals * kRow];
+    const bool general = pr.general || __ldcg(fv.flag) == fv.epoch;
+    if (general)
+        load_rows(rows, t.dw);
+    const Group<LANES> g;
+    const size_t i = g.i;
+    if (i >= n)
+        return;
+    double B[D * D];
+#pragma unroll
+    for (int a = 0; a < D * D; ++a)
+        B[a] = f.B[a * n + i];
+    const double beta = k.slope * k.inv_c0_ave;
+    double div = 0, pd[3] = {0, 0, 0};
+    if (general)
+    {
+        double v_i[3] = {0, 0, 0}, x_i[3], r[3], e[3], du[3], be[3], inv;
+        load_point<D>(f.vel, n, i, v_i);
+        load_point<D>(f.pos, n, i, x_i);
+        for_each_neighbor(in, g, [&](uint32_t j) {
+            const double n2 = separation<D>(x_i, f.pos, n, j, r, inv);
+            const double dWV = tabulated(rows, (n2 * inv) * t.inv_step) * f.Vol[j];
+#pragma unroll
+            for (int a = 0; a < D; ++a)
+            {
+                e[a] = r[a] * inv;
+                du[a] = v_i[a] - f.vel[a * n + j];
+            }
+            corrected<D>(B, e, be);
+            div = fma(dot<D>(du, be), dWV, div);
+            const double pj = limited_jump(beta, dot<D>(du, e), dWV);
+#pragma unroll
+            for (int a = 0; a < D; ++a)
+                pd[a] = fma(pj, e[a], pd[a]);
+        });
+        div = g.sum(div);
+#pragma unroll
+        for (int a = 0; a < D; ++a)
+            pd[a] = g.sum(pd[a]);
+    }
+    else
+    {
+        ck_fixed_2nd<D, LANES>(n, g, pr, fv, volume_unit(f.Vol), B, 1.0 / beta, pd, &div);
+        div *= pr.factor;
+#pragma unroll
+        for (int a = 0; a < D; ++a)
+            pd[a] *= pr.factor * beta;
+    }
+    if (!g.leads())
+        return;
+    if (wall_count && wall_count[i] > 0)
+    {
+        div += wall_sum[D * n + i];
+#pragma unroll
+        for (int a = 0; a < D; ++a)
+            pd[a] += wall_sum[a * n + i];
+    }
     const double comp_i = f.compression[i], Vol_i = f.Vol[i];
     const double rate = f.rate[i] + div * comp_i;
     f.rate[i] = rate;
@@ -640,7 +1078,7 @@ __global__ void __launch_bounds__(kBlock) k_ck_second(size_t n, CKFluid f, CKWal
     for (int a = 0; a < D; ++a)
     {
         f.force[a * n + i] = pd[a] * k.rho0c0_geo_ave * Vol_i;
-        f.dpos[a * n + i] += v_i[a] * dt * 0.5;
+        f.dpos[a * n + i] += f.vel[a * n + i] * dt * 0.5;
     }
     const double comp = comp_i + 0.5 * dt * rate;
     f.compression[i] = comp;
@@ -972,6 +1410,56 @@ int sweep_lanes(sphx_ctx ctx, int dim, size_t n)
         SPHX_LAUNCHED((b)->ctx);                                                                                       \
     } while (0)
 
+// The pair geometry of the relation's current lists, made on the first half step after an
+// update, and the record buffer of a half step with a fresh epoch for its verdict.
+static int ck_pairs(sphx_relation rel, const CKFluid &f, const TabK &t, const CKParams &k, int half, CKPairs &pr,
+                    fx::Fixed &fixed)
+{
+    sphx_ctx ctx = rel->ctx;
+    const int D = rel->src->dim;
+    const size_t n = rel->n_src, slots = size_t(rel->cap) * n;
+    if (!rel->ck_rec)
+    {
+        SPHX_CUDA(cudaMalloc(&rel->ck_pos, n * D * sizeof(double)));
+        SPHX_CUDA(cudaMalloc(&rel->ck_value, n * Rec1<3>::words * sizeof(long long)));
+        if (D == 2)
+            SPHX_CUDA(cudaMalloc(&rel->ck_k, slots * sizeof(int2)));
+        SPHX_CUDA(cudaMalloc(&rel->ck_rec, slots * (D == 2 ? 1 : 2) * sizeof(int4)));
+        rel->ck_version = 0;
+    }
+    pr = CKPairs{rel->count, rel->j, fx::EntryStore{rel->ck_rec, rel->ck_k}, unsigned(rel->cap),
+                 uint32_t(rel->tgt->n), wendland(D, rel->h).factor_dW, rel->ck_pos,
+                 rel->cap > int(fx::kMaxCap) || !(k.slope * k.inv_c0_ave >= 0.0)};
+    if (rel->ck_version != rel->version)
+    {
+        const double inv_factor = 1.0 / pr.factor;
+        CK_SWEEP(k_ck_pairs, D, ctx, n, n, f.pos, lists_of(rel), t, inv_factor, pr.at, rel->ck_pos);
+        rel->ck_version = rel->version;
+    }
+    fixed = fx::Fixed{rel->ck_value, rel->fx_flag + half, ++rel->fx_epoch[half],
+                      reinterpret_cast<unsigned long long *>(rel->fx_flag + 4)};
+    return SPHX_OK;
+}
+
+// The wall terms of a half step, into the contact relation's workspace.
+template <int HALF>
+static int ck_wall_terms(sphx_relation wall, const CKFluid &f, const CKWall &w, const TabK &t, const CKParams &k)
+{
+    if (!wall || wall->n_active == 0)
+        return SPHX_OK;
+    sphx_ctx ctx = wall->ctx;
+    const size_t n = wall->src->n, na = wall->n_active;
+    const unsigned grid = grid_for(na * kWallLanes, kBlock);
+    if (wall->src->dim == 2)
+        k_ck_wall<2, HALF><<<grid, kBlock, 0, ctx->stream>>>(n, na, wall->active, f, w, lists_of(wall), t, k,
+                                                             wall->contact_sum);
+    else
+        k_ck_wall<3, HALF><<<grid, kBlock, 0, ctx->stream>>>(n, na, wall->active, f, w, lists_of(wall), t, k,
+                                                             wall->contact_sum);
+    SPHX_LAUNCHED(ctx);
+    return SPHX_OK;
+}
+
 extern "C" int sphx_ck_density_regularization(sphx_relation inner, sphx_relation wall, const sphx_fluid_params *p)
 {
     SPHX_TRY(ck_check(inner, wall));
@@ -1108,9 +1596,14 @@ extern "C" int sphx_ck_acoustic_step_1st_half(sphx_relation inner, sphx_relation
     if (n == 0)
         return SPHX_OK;
     CKParams k = make_ck_params(*p);
-    CK_DISPATCH(b, k_ck_init1, grid_for(n, kBlock), n, f, k, dt);
-    CK_SWEEP(k_ck_interact1, b->dim, b->ctx, n, n, f, w, lists_of(inner), lists_of(wall),
-                make_tab(b->dim, inner->h), k, dt);
+    const TabK t = make_tab(b->dim, inner->h);
+    CKPairs pr{};
+    fx::Fixed fp{};
+    SPHX_TRY(ck_pairs(inner, f, t, k, 0, pr, fp));
+    CK_DISPATCH(b, k_ck_init1, grid_for(n, kBlock), n, f, k, dt, pr, fp);
+    SPHX_TRY((ck_wall_terms<1>(wall, f, w, t, k)));
+    CK_SWEEP(k_ck_interact1, b->dim, b->ctx, n, n, f, lists_of(inner), pr, fp, t, k, dt,
+             wall ? wall->count : nullptr, wall ? wall->contact_sum : nullptr);
     return SPHX_OK;
 }
 
@@ -1128,8 +1621,21 @@ extern "C" int sphx_ck_acoustic_step_2nd_half(sphx_relation inner, sphx_relation
     size_t n = b->n;
     if (n == 0)
         return SPHX_OK;
-    CK_SWEEP(k_ck_second, b->dim, b->ctx, n, n, f, w, lists_of(inner), lists_of(wall),
-                make_tab(b->dim, inner->h), make_ck_params(*p), dt);
+    CKParams k = make_ck_params(*p);
+    const TabK t = make_tab(b->dim, inner->h);
+    sphx_ctx ctx = b->ctx;
+    CKPairs pr{};
+    fx::Fixed fv{};
+    SPHX_TRY(ck_pairs(inner, f, t, k, 1, pr, fv));
+    if (b->dim == 2)
+        fx::k_largest_velocity<2><<<red_grid(ctx, n), kBlock, 0, ctx->stream>>>(n, f.vel, fv);
+    else
+        fx::k_largest_velocity<3><<<red_grid(ctx, n), kBlock, 0, ctx->stream>>>(n, f.vel, fv);
+    SPHX_LAUNCHED(ctx);
+    CK_DISPATCH(b, k_ck_init2, grid_for(n, kBlock), n, f, pr, fv);
+    SPHX_TRY((ck_wall_terms<2>(wall, f, w, t, k)));
+    CK_SWEEP(k_ck_second, b->dim, ctx, n, n, f, lists_of(inner), pr, fv, t, k, dt, wall ? wall->count : nullptr,
+             wall ? wall->contact_sum : nullptr);
     return SPHX_OK;
 }
 

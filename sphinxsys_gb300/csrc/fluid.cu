@@ -22,6 +22,8 @@
 #include "sphx_internal.cuh"
 
 using namespace sphx;
+using fx::Fixed;
+using fx::velocity_unit;
 
 namespace
 {
@@ -105,23 +107,6 @@ InnerPairs pairs_of(sphx_relation r)
     return nb;
 }
 
-// The fixed-point particle values of one sweep and its verdict: *flag == epoch when the
-// kernel that made them found a value outside the range of the format.
-struct Fixed
-{
-    long long *value; // pressure: 1 word a particle; velocity: 2 (2D) or 4 (3D) words
-    uint32_t *flag;
-    uint32_t epoch;
-    unsigned long long *speed; // epoch and the largest binary exponent of a velocity component
-};
-
-// The unit 2^k of the velocities: their largest component takes 60 bits.
-__device__ __forceinline__ int velocity_unit(const Fixed &f)
-{
-    const int e = int(__ldcg(f.speed) & 0x7ffull);
-    return max(e, 600) - 1022 - fx::kVelocityBits;
-}
-
 struct FluidVars
 {
     double *pos, *vel, *force;
@@ -172,25 +157,6 @@ __global__ void k_init_1st(size_t n, double *__restrict__ rho, const double *__r
         *fp.flag = fp.epoch;
 }
 
-template <int D>
-__global__ void k_largest_velocity(size_t n, const double *__restrict__ vel, Fixed fv)
-{
-    int m = 0;
-    for (size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n * D; i += size_t(gridDim.x) * blockDim.x)
-        m = max(m, __double2hiint(vel[i]) & 0x7fffffff);
-    m = __reduce_max_sync(0xffffffffu, m);
-    __shared__ int sm[32];
-    if ((threadIdx.x & 31u) == 0)
-        sm[threadIdx.x >> 5] = m;
-    __syncthreads();
-    if (threadIdx.x != 0)
-        return;
-    for (unsigned k = 1; k < (blockDim.x >> 5); ++k)
-        m = max(m, sm[k]);
-    // the epoch in front makes the value of every earlier call smaller
-    atomicMax(fv.speed, static_cast<unsigned long long>(fv.epoch) << 11 | unsigned(m >> 20));
-}
-
 // Velocities in fixed point, one record of 16 (2D) or 32 (3D) bytes a particle; converted by
 // integer instructions on the bits (the FP64 form of this pass took 47 us for 1,702,400
 // particles, three times its memory traffic).
@@ -201,7 +167,7 @@ __global__ void k_init_2nd(size_t n, const double *__restrict__ vel, const doubl
     if (i >= n)
         return;
     const int unit = velocity_unit(fv);
-    bool fits = __double_as_longlong(Vol[i]) == __double_as_longlong(Vol[0]) && unit < 400;
+    bool fits = __double_as_longlong(Vol[i]) == __double_as_longlong(Vol[0]) && unit < 200;
     long long q[4] = {0, 0, 0, 0};
 #pragma unroll
     for (int d = 0; d < D; ++d)
@@ -491,12 +457,6 @@ __device__ __forceinline__ void value_1st(const SweepSums<D> &s, double *force, 
         force[d] = s.force[d].value() * unit;
 }
 
-// A speed of `t` units at alignment 0 in the units of alignment a; 2^57 is above every speed.
-__device__ __forceinline__ long long limit_at(long long t, int a)
-{
-    return t < (1ll << (57 - a)) ? t << a : 1ll << 57;
-}
-
 // Integration2ndHalf in fixed point, u = (v_i - v_j) . e: R = sum u K and
 // F = sum u min(u+, u_lim) K e, the dissipation without its constant factors; u_lim is the
 // speed at which the limiter reaches 1.
@@ -554,12 +514,12 @@ __device__ __forceinline__ void fixed_2nd(size_t n, size_t i, unsigned sub, cons
         {
             first = false;
             al.start(top);
-            lim = limit_at(t_lim, al.a);
+            lim = fx::limit_at(t_lim, al.a);
         }
         while (al.over(top))
         {
             const int k = al.step();
-            lim = limit_at(t_lim, al.a);
+            lim = fx::limit_at(t_lim, al.a);
             R.shift(k);
 #pragma unroll
             for (int d = 0; d < D; ++d)
@@ -569,20 +529,9 @@ __device__ __forceinline__ void fixed_2nd(size_t n, size_t i, unsigned sub, cons
         for (int u = 0; u < U; ++u)
         {
             const int2 K = q[u].k;
-            const long long T = al.apply(hh[u], m[u]); // u
-            const int th = int(T >> 31), tl = int(unsigned(T) & 0x7fffffffu);
-            // u K in units of 2^57
-            const long long wm = fx::low_product(tl, K.y, fx::mad(tl, K.x, fx::mad(th, K.y, 1 << 25)));
-            const long long w = (fx::mad(th, K.x, 0) << 5) + (wm >> 26);
+            long long w, sc;
+            fx::jump(al.apply(hh[u], m[u]), K, lim, &w, &sc);
             R.m += w;
-            // min(u+, limit)
-            const bool capped = T > lim;
-            const int bh = capped ? int(lim >> 31) : max(th, 0);
-            const int bl = capped ? int(unsigned(lim) & 0x7fffffffu) : (th < 0 ? 0 : tl);
-            const int ah = int(w >> 31), av = int(unsigned(w) & 0x7fffffffu);
-            // in units of 2^53
-            const long long sm = fx::low_product(av, bl, fx::mad(av, bh, fx::mad(ah, bl, 1 << 21)));
-            const long long sc = (fx::mad(ah, bh, 0) << 9) + (sm >> 22);
             const int sh = int(sc >> 31), sl = int(unsigned(sc) & 0x7fffffffu);
 #pragma unroll
             for (int d = 0; d < D; ++d)
@@ -1312,9 +1261,9 @@ extern "C" int sphx_integration_2nd_half_with_wall_riemann(sphx_relation inner, 
     sphx_ctx ctx = b->ctx;
     const Fixed fv = fixed_of(inner, 1);
     if (b->dim == 2)
-        k_largest_velocity<2><<<reduce_grid(ctx, n), kBlock, 0, ctx->stream>>>(n, f.vel, fv);
+        fx::k_largest_velocity<2><<<reduce_grid(ctx, n), kBlock, 0, ctx->stream>>>(n, f.vel, fv);
     else
-        k_largest_velocity<3><<<reduce_grid(ctx, n), kBlock, 0, ctx->stream>>>(n, f.vel, fv);
+        fx::k_largest_velocity<3><<<reduce_grid(ctx, n), kBlock, 0, ctx->stream>>>(n, f.vel, fv);
     SPHX_LAUNCHED(ctx);
     if (b->dim == 2)
         k_init_2nd<2><<<grid_for(n, 256), 256, 0, ctx->stream>>>(n, f.vel, f.Vol, fv);

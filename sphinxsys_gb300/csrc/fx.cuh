@@ -165,6 +165,29 @@ struct Align
     }
 };
 
+// A speed of `t` units at alignment 0 in the units of alignment a; 2^57 is above every speed.
+__device__ __forceinline__ long long limit_at(long long t, int a)
+{
+    return t < (1ll << (57 - a)) ? t << a : 1ll << 57;
+}
+
+// The dissipative jump of a pair: u of alignment a, K its weight: u K in units of 2^57 and
+// u K min(u+, lim) in units of 2^53.
+__device__ __forceinline__ void jump(long long u, int2 K, long long lim, long long *uK, long long *sc)
+{
+    const int th = int(u >> 31), tl = int(unsigned(u) & 0x7fffffffu);
+    const long long wm = low_product(tl, K.y, mad(tl, K.x, mad(th, K.y, 1 << 25)));
+    const long long w = (mad(th, K.x, 0) << 5) + (wm >> 26);
+    if (uK)
+        *uK = w;
+    const bool capped = u > lim;
+    const int bh = capped ? int(lim >> 31) : max(th, 0);
+    const int bl = capped ? int(unsigned(lim) & 0x7fffffffu) : (th < 0 ? 0 : tl);
+    const int ah = int(w >> 31), av = int(unsigned(w) & 0x7fffffffu);
+    const long long sm = low_product(av, bl, mad(av, bh, mad(ah, bl, 1 << 21)));
+    *sc = (mad(ah, bh, 0) << 9) + (sm >> 22);
+}
+
 // The list entries of an inner relation: kernel derivative over its prefactor and unit
 // vector.  3D: one record of 32 bytes {K, e} a slot; 2D: {e} of 16 bytes, K in its own array.
 template <int D>
@@ -333,5 +356,42 @@ __device__ __forceinline__ void group_sum(Sum &s)
         s.m = group_sum<LANES>(s.m);
     }
 }
+// ---------------------------------------------------------------- particle values
+// The fixed-point particle values of one sweep and its verdict: *flag == epoch when the
+// kernel that made them found a value outside the range of the format.
+struct Fixed
+{
+    long long *value; // pressure: 1 word a particle; velocity: 2 (2D) or 4 (3D) words
+    uint32_t *flag;
+    uint32_t epoch;
+    unsigned long long *speed; // epoch and the largest binary exponent of a velocity component
+};
+
+// The unit 2^k of the velocities: their largest component takes 60 bits.
+__device__ __forceinline__ int velocity_unit(const Fixed &f)
+{
+    const int e = int(__ldcg(f.speed) & 0x7ffull);
+    return max(e, 700) - 1022 - kVelocityBits;
+}
+
+template <int D>
+static __global__ void k_largest_velocity(size_t n, const double *__restrict__ vel, Fixed fv)
+{
+    int m = 0;
+    for (size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n * D; i += size_t(gridDim.x) * blockDim.x)
+        m = max(m, __double2hiint(vel[i]) & 0x7fffffff);
+    m = __reduce_max_sync(0xffffffffu, m);
+    __shared__ int sm[32];
+    if ((threadIdx.x & 31u) == 0)
+        sm[threadIdx.x >> 5] = m;
+    __syncthreads();
+    if (threadIdx.x != 0)
+        return;
+    for (unsigned k = 1; k < (blockDim.x >> 5); ++k)
+        m = max(m, sm[k]);
+    // the epoch in front makes the value of every earlier call smaller
+    atomicMax(fv.speed, static_cast<unsigned long long>(fv.epoch) << 11 | unsigned(m >> 20));
+}
+
 } // namespace fx
 } // namespace sphx

@@ -425,6 +425,15 @@ void sphx_relation_s::release()
     cudaFree(r);
     cudaFree(e);
     cudaFree(wsum);
+    cudaFree(ck_rec);
+    cudaFree(ck_k);
+    cudaFree(ck_pos);
+    cudaFree(ck_value);
+    ck_rec = nullptr;
+    ck_k = nullptr;
+    ck_pos = nullptr;
+    ck_value = nullptr;
+    ck_version = 0;
     cudaFree(fx_rec);
     cudaFree(fx_k);
     cudaFree(active);
@@ -649,6 +658,7 @@ extern "C" int sphx_relation_update(sphx_relation rel)
     if (rel->cl->n != rel->tgt->n)
         return fail(SPHX_ERR_INVALID_ARG, "target cell list holds %zu particles but the target body has %zu; update "
                                           "the cell linked list first", rel->cl->n, rel->tgt->n);
+    ++rel->version;
     sphx_ctx ctx = rel->ctx;
     size_t n = rel->src->n;
     if (rel->cap == 0 || rel->n_src != n)

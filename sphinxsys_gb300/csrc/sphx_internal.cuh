@@ -171,6 +171,13 @@ struct sphx_relation_s
     uint32_t fx_epoch[3] = {0, 0, 0};
     longlong4_32a *fx_pos = nullptr; // cell-list entries: position in fixed point, particle
     size_t fx_pos_cap = 0;
+    // CK methods (ck.cu): the tabulated kernel derivative and unit vector of the pairs of list
+    // `ck_version`, made from the positions ck_pos, and the particle records of a sweep
+    uint64_t version = 0, ck_version = 0;
+    int4 *ck_rec = nullptr;
+    int2 *ck_k = nullptr;
+    double *ck_pos = nullptr;
+    long long *ck_value = nullptr;
     int reserve_positions(size_t n);
     // Contact relations: the source particles with neighbours (n_active of them, in no
     // order) and a workspace for their sums.
