@@ -129,8 +129,8 @@ class BatchDamBreak:
     def download(self, instance: int):
         """(position, velocity, density, pressure) of one instance in its input order."""
         n, d = self.n_fluid[instance], self.dim
-        pos, vel = np.zeros((n, d)), np.zeros((n, d))
-        rho, p = np.zeros(n), np.zeros(n)
+        pos, vel = np.empty((n, d)), np.empty((n, d))
+        rho, p = np.empty(n), np.empty(n)
         N.call("sphx_batch_download", self.handle, int(instance), S._dptr(pos), S._dptr(vel), S._dptr(rho),
                S._dptr(p))
         return pos, vel, rho, p
