@@ -16,21 +16,21 @@
 //
 // Pair geometry comes from the current Position, which the CK loop moves once per
 // advection step (UpdateParticlePosition); the neighbour index lists are the relations'
-// (the cut-off test of the configuration).  Every sum runs in list order, so results match
-// the oracle's restatement to rounding.  Fusion: the 1st half is two launches
-// (compression / density / pressure / displacement initialisation, then interaction + wall
-// + velocity update), the 2nd half one launch (displacement, interaction, wall, compression
-// update): each fused update touches only the particle's own variables, which no other
-// particle reads in that interaction.
+// (the cut-off test of the configuration).  Sums agree with the oracle's list-order sums to
+// rounding; a particle's list is shared by up to 8 threads.
 //
-// Bound: the FP64 pipe (2 lanes a cycle per SM on GB300), so the once-per-step sums are
-// written for few FP64 instructions a pair: one reciprocal square root for distance and
-// direction, the table as polynomial coefficients (3 fused multiply-adds; its Lagrange form
-// takes 5 divisions), factors common to a particle's pairs applied to the sums.  The half
-// steps keep the pair geometry between relation updates and sum in fixed point.  One
-// advection step of the 3D dam break at dp = 0.02 (90,000 particles): 35.2 ms, 10.0 with the
-// lighter FP64 sums, 4.7 with the fixed-point half steps (a 1st / 2nd half 0.70 / 0.87 ->
-// 0.13 / 0.18 ms); error against 64-bit references 2.2e-13, 1.9e-13, 1.9e-13.
+// Bound: the FP64 pipe (2 lanes a cycle per SM on GB300), so the FP64 sums are written for
+// few instructions a pair: one reciprocal square root for distance and direction, the table
+// as polynomial coefficients (3 fused multiply-adds; its Lagrange form takes 5 divisions),
+// factors common to a particle's pairs applied to the sums.  The pair geometry is formed once
+// per relation update, in the pass of the compression sum, and the inner sums of the
+// correction matrix, the free-surface indication and the half steps run in fixed point on it;
+// wall terms go to their own kernels over the particles that have any.  One advection step of
+// the 3D dam break at dp = 0.02 (90,000 particles): 35.0 ms, 10.0 with the lighter FP64 sums,
+// 4.8 with the fixed-point half steps (a 1st / 2nd half 0.70 / 0.87 -> 0.14 / 0.14 ms and
+// 0.07 ms for the walls), 3.9 with the other sums from the kept geometry (correction 0.58 ->
+// 0.20 ms, indication sums 0.37 -> 0.10 ms, geometry and compression sum 0.31 + 0.34 ->
+// 0.44 ms; device times of single launches).
 #include <algorithm>
 #include <cmath>
 #include <string>
@@ -295,11 +295,10 @@ __device__ __forceinline__ double limited_jump(double beta, double u, double w)
 }
 
 // ---------------------------------------------------------------- kernels
-// CompressionSummation<Inner, Contact> and, with REGULARIZE, the post-state
-// DensityRegularization<FreeSurface> in the same pass.
-template <int D, int LANES, bool REGULARIZE>
-__device__ __forceinline__ void ck_summation(size_t n, const CKFluid &f, const CKWall &w, const Lists &in,
-                                             const Lists &wl, const TabK &t, double rho0)
+// CompressionSummation<Inner, Contact>.
+template <int D, int LANES>
+__global__ void __launch_bounds__(kBlock)
+    k_ck_compression_summation(size_t n, CKFluid f, CKWall w, Lists in, Lists wl, TabK t)
 {
     __shared__ double rows[kIntervals * kRow];
     load_rows(rows, t.w);
@@ -319,30 +318,8 @@ __device__ __forceinline__ void ck_summation(size_t n, const CKFluid &f, const C
             sum = fma(tabulated(rows, (n2 * inv) * t.inv_step), w.Vol_ref[j], sum);
         });
     sum = g.sum(sum);
-    if (!g.leads())
-        return;
-    sum += t.W0 * f.Vol_ref[i];
-    f.csum[i] = sum;
-    if (REGULARIZE)
-    {
-        double comp = fmax(sum, 1.0);
-        f.compression[i] = comp;
-        f.rho[i] = comp * rho0;
-    }
-}
-
-template <int D, int LANES>
-__global__ void __launch_bounds__(kBlock)
-    k_ck_regularization(size_t n, CKFluid f, CKWall w, Lists in, Lists wl, TabK t, double rho0)
-{
-    ck_summation<D, LANES, true>(n, f, w, in, wl, t, rho0);
-}
-
-template <int D, int LANES>
-__global__ void __launch_bounds__(kBlock)
-    k_ck_compression_summation(size_t n, CKFluid f, CKWall w, Lists in, Lists wl, TabK t, double rho0)
-{
-    ck_summation<D, LANES, false>(n, f, w, in, wl, t, rho0);
+    if (g.leads())
+        f.csum[i] = fma(t.W0, f.Vol_ref[i], sum);
 }
 
 // DensityRegularization<SPHBody, WeaklyCompressibleFluid, FreeSurface> alone
@@ -410,67 +387,6 @@ __device__ __forceinline__ void inverse(const double *A, double *R)
     R[8] = (A[0] * A[4] - A[1] * A[3]) / d;
 }
 
-// The sum over r_a dW e_b V_j is symmetric (e = r / |r|): its upper half is accumulated.
-template <int D, int LANES>
-__global__ void __launch_bounds__(kBlock)
-    k_ck_correction(size_t n, CKFluid f, CKWall w, Lists in, Lists wl, TabK t, double alpha)
-{
-    __shared__ double rows[kIntervals * kRow];
-    load_rows(rows, t.dw);
-    const Group<LANES> g;
-    const size_t i = g.i;
-    if (i >= n)
-        return;
-    double B[D * D];
-    for (int k = 0; k < D * D; ++k)
-        B[k] = 0.0;
-    double x_i[3], r[3], inv;
-    load_point<D>(f.pos, n, i, x_i);
-    auto add = [&](double n2, double Vj) {
-        const double k = (tabulated(rows, (n2 * inv) * t.inv_step) * Vj) * inv;
-#pragma unroll
-        for (int a = 0; a < D; ++a)
-        {
-            const double ka = k * r[a];
-#pragma unroll
-            for (int b = a; b < D; ++b)
-                B[a * D + b] -= ka * r[b];
-        }
-    };
-    for_each_neighbor(in, g, [&](uint32_t j) { add(separation<D>(x_i, f.pos, n, j, r, inv), f.Vol[j]); });
-    if (wl.J)
-        for_each_neighbor(wl, g, [&](uint32_t j) { add(separation<D>(x_i, w.pos, w.nw, j, r, inv), w.Vol[j]); });
-#pragma unroll
-    for (int a = 0; a < D; ++a)
-#pragma unroll
-        for (int b = a; b < D; ++b)
-            B[b * D + a] = B[a * D + b] = g.sum(B[a * D + b]);
-    if (!g.leads())
-        return;
-    double determinant = det<D>(B);
-    double det_sqr = fmax(alpha - determinant, 0.0);
-    // inverseTikhonov (vector_functions.h:199-203): (B^T B + eps I)^-1 B^T, eps = SqrtEps
-    double BtB[D * D], Inv[D * D];
-    for (int a = 0; a < D; ++a)
-        for (int b = 0; b < D; ++b)
-        {
-            double sum = 0;
-            for (int k = 0; k < D; ++k)
-                sum += B[k * D + a] * B[k * D + b];
-            BtB[a * D + b] = sum + (a == b ? 1.0e-8 : 0.0);
-        }
-    inverse<D>(BtB, Inv);
-    double weight = determinant / (determinant + det_sqr);
-    for (int a = 0; a < D; ++a)
-        for (int b = 0; b < D; ++b)
-        {
-            double sum = 0;
-            for (int k = 0; k < D; ++k)
-                sum += Inv[a * D + k] * B[b * D + k];
-            f.B[(a * D + b) * n + i] = weight * sum + (1.0 - weight) * (a == b ? 1.0 : 0.0);
-        }
-}
-
 // ---------------------------------------------------------------- acoustic half steps
 // The pair geometry does not change between relation updates while the particles stay where
 // they were, so the tabulated kernel derivative and the unit vector of every pair are formed
@@ -496,21 +412,26 @@ struct CKPairs
     uint32_t limit;
     double factor; // of the tabulated derivative
     const double *pos; // positions the entries were made from
+    const int2 *r;     // distances over 2 h
     bool general;      // lists or parameters the integer sums cannot take
 };
 
-template <int D, int LANES>
-__global__ void __launch_bounds__(kBlock) k_ck_pairs(size_t n, const double *__restrict__ pos, Lists in, TabK t,
-                                                     double inv_factor, fx::EntryStore at, double *__restrict__ copy)
+// SUM: with the inner part of CompressionSummation in the same pass.
+template <int D, int LANES, bool SUM>
+__device__ __forceinline__ void make_pairs(size_t n, const CKFluid &f, const Lists &in, const TabK &t, double inv_factor,
+                                           double inv_cutoff, const fx::EntryStore &at, int2 *out_r, double *copy)
 {
-    __shared__ double rows[kIntervals * kRow];
+    __shared__ double rows[kIntervals * kRow], wrows[SUM ? kIntervals * kRow : 1];
     load_rows(rows, t.dw);
+    if (SUM)
+        load_rows(wrows, t.w);
     const Group<LANES> g;
     const size_t i = g.i;
     if (i >= n)
         return;
-    double x_i[3], r[3], inv;
-    load_point<D>(pos, n, i, x_i);
+    double x_i[3], r[3], inv, sum = 0.0;
+    int far = 0;
+    load_point<D>(f.pos, n, i, x_i);
     const unsigned c = min(in.count[i], in.cap);
     for (unsigned s = g.sub; s < c; s += LANES)
     {
@@ -518,18 +439,44 @@ __global__ void __launch_bounds__(kBlock) k_ck_pairs(size_t n, const double *__r
         const uint32_t j = in.J[slot];
         if (!entry_ok(in, j))
             continue;
-        const double n2 = separation<D>(x_i, pos, n, j, r, inv);
-        fx::Entry<D> q;
-        q.k = fx::encode(tabulated(rows, (n2 * inv) * t.inv_step) * inv_factor);
+        const double n2 = separation<D>(x_i, f.pos, n, j, r, inv);
+        const double len = n2 * inv, q = len * t.inv_step, rr = len * inv_cutoff;
+        fx::Entry<D> e;
+        e.k = fx::encode(tabulated(rows, q) * inv_factor);
 #pragma unroll
         for (int a = 0; a < D; ++a)
-            q.e[a] = fx::encode(r[a] * inv);
-        at.store<D>(slot, q);
+            e.e[a] = fx::encode(r[a] * inv);
+        at.store<D>(slot, e);
+        out_r[slot] = fx::encode(rr);
+        far |= !(rr < 1.5);
+        if (SUM)
+            sum = fma(tabulated(wrows, q), f.Vol_ref[j], sum);
     }
-    if (g.leads())
+    far = fx::group_sum<LANES>(far);
+    if (SUM)
+        sum = g.sum(sum);
+    if (!g.leads())
+        return;
+    // a pair the format cannot hold (the particles left their list): no position matches
 #pragma unroll
-        for (int a = 0; a < D; ++a)
-            copy[a * n + i] = x_i[a];
+    for (int a = 0; a < D; ++a)
+        copy[a * n + i] = far ? __longlong_as_double(0x7ff8000000000001ll) : x_i[a];
+    if (SUM)
+        f.csum[i] = fma(t.W0, f.Vol_ref[i], sum);
+}
+template <int D, int LANES>
+__global__ void __launch_bounds__(kBlock)
+    k_ck_pairs(size_t n, CKFluid f, Lists in, TabK t, double inv_factor, double inv_cutoff, fx::EntryStore at,
+               int2 *__restrict__ out_r, double *__restrict__ copy)
+{
+    make_pairs<D, LANES, false>(n, f, in, t, inv_factor, inv_cutoff, at, out_r, copy);
+}
+template <int D, int LANES>
+__global__ void __launch_bounds__(kBlock)
+    k_ck_pairs_sum(size_t n, CKFluid f, Lists in, TabK t, double inv_factor, double inv_cutoff, fx::EntryStore at,
+                   int2 *__restrict__ out_r, double *__restrict__ copy)
+{
+    make_pairs<D, LANES, true>(n, f, in, t, inv_factor, inv_cutoff, at, out_r, copy);
 }
 
 template <int D>
@@ -932,6 +879,29 @@ __global__ void __launch_bounds__(kBlock) k_ck_wall(size_t n, size_t n_active, c
     sum[D * n + i] = q;
 }
 
+// The wall part of CompressionSummation, added to the inner part.
+template <int D>
+__global__ void __launch_bounds__(kBlock) k_ck_wall_summation(size_t n, size_t n_active,
+                                                              const uint32_t *__restrict__ active, CKFluid f, CKWall w,
+                                                              Lists wl, TabK t)
+{
+    __shared__ double rows[kIntervals * kRow];
+    load_rows(rows, t.w);
+    Group<kWallLanes> g;
+    if (g.i >= n_active)
+        return;
+    g.i = active[g.i];
+    double x_i[3], r[3], inv, sum = 0.0;
+    load_point<D>(f.pos, n, g.i, x_i);
+    for_each_neighbor(wl, g, [&](uint32_t j) {
+        const double n2 = separation<D>(x_i, w.pos, w.nw, j, r, inv);
+        sum = fma(tabulated(rows, (n2 * inv) * t.inv_step), w.Vol_ref[j], sum);
+    });
+    sum = g.sum(sum);
+    if (g.leads())
+        f.csum[g.i] += sum;
+}
+
 // AverageP of both corrections: sum_j (p_i B_j + p_j B_i) e dW V_j =
 // p_i sum_j (B_j e) dW V_j + B_i sum_j p_j e dW V_j, so the pair needs one matrix product.
 template <int D, int LANES>
@@ -1085,6 +1055,226 @@ __global__ void __launch_bounds__(kBlock, 4)
     f.rho[i] = comp * k.rho0;
 }
 
+// ---------------------------------------------------------------- once per step
+// Volumes in fixed point for the sums below, with the verdict on positions and volumes.
+template <int D>
+__global__ void k_ck_volumes(size_t n, CKFluid f, CKPairs pr, fx::Fixed fp)
+{
+    const size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
+    if (i >= n)
+        return;
+    bool fits = stayed<D>(f.pos, pr.pos, n, i) && abs(volume_unit(f.Vol)) < 250;
+    const long long v = fx::fixed(f.Vol[i], volume_unit(f.Vol), fits);
+    fits = fits && v >= 0 && v < (1ll << fx::kListBits);
+    fp.value[i] = v;
+    if (!fits)
+        *fp.flag = fp.epoch;
+}
+
+// K V_j r / (2 h) of a pair in units of 2^(unit of the volumes - 3).
+__device__ __forceinline__ long long moment(int2 K, long long V, int2 r)
+{
+    const int2 kv = weighted(K, V);
+    const fx::Halves k{kv.x, kv.y}, q{r.x, r.y};
+    return (fx::mad(k.h, q.h, 0) << 8) + (fx::middle(k, q, 1 << 22) >> 23);
+}
+
+// sum_j r_a dW V_j e_b = sum_j (|r| dW V_j) e_a e_b, symmetric: its upper half, into the matrix
+// array (the final matrix replaces it, k_ck_correction_finish).
+template <int D, int LANES>
+__global__ void __launch_bounds__(kBlock)
+    k_ck_correction_sums(size_t n, CKFluid f, Lists in, CKPairs pr, fx::Fixed fp, TabK t, double cutoff)
+{
+    __shared__ double rows[kIntervals * kRow];
+    const bool general = pr.general || __ldcg(fp.flag) == fp.epoch;
+    if (general)
+        load_rows(rows, t.dw);
+    const Group<LANES> g;
+    const size_t i = g.i;
+    if (i >= n)
+        return;
+    if (general)
+    {
+        double B[D * D], x_i[3], r[3], inv;
+        for (int k = 0; k < D * D; ++k)
+            B[k] = 0.0;
+        load_point<D>(f.pos, n, i, x_i);
+        for_each_neighbor(in, g, [&](uint32_t j) {
+            const double n2 = separation<D>(x_i, f.pos, n, j, r, inv);
+            const double k = (tabulated(rows, (n2 * inv) * t.inv_step) * f.Vol[j]) * inv;
+#pragma unroll
+            for (int a = 0; a < D; ++a)
+            {
+                const double ka = k * r[a];
+#pragma unroll
+                for (int b = a; b < D; ++b)
+                    B[a * D + b] = fma(ka, r[b], B[a * D + b]);
+            }
+        });
+#pragma unroll
+        for (int a = 0; a < D; ++a)
+#pragma unroll
+            for (int b = a; b < D; ++b)
+            {
+                const double v = g.sum(B[a * D + b]);
+                if (g.leads())
+                    f.B[(a * D + b) * n + i] = v;
+            }
+        return;
+    }
+    fx::Sum M[D * D];
+    int folded = 0;
+    const unsigned cnt = min(pr.count[i], pr.cap);
+    for (unsigned s = g.sub; s < cnt; s += LANES)
+    {
+        const size_t slot = size_t(s) * n + i;
+        const uint32_t j = pr.J[slot];
+        if (!entry_ok(in, j))
+            continue;
+        const fx::Entry<D> q = pr.at.load<D>(slot);
+        const fx::Halves x = fx::halves(moment(q.k, __ldg(fp.value + j), pr.r[slot]));
+#pragma unroll
+        for (int a = 0; a < D; ++a)
+        {
+            const fx::Halves e{q.e[a].x, q.e[a].y};
+            const fx::Halves y = fx::halves((fx::mad(x.h, e.h, 0) << 5) + (fx::middle(x, e, 1 << 25) >> 26));
+#pragma unroll
+            for (int b = a; b < D; ++b)
+                M[a * D + b].add(y.h, y.l, q.e[b]);
+        }
+        if (++folded == fx::kFold)
+        {
+            folded = 0;
+#pragma unroll
+            for (int a = 0; a < D; ++a)
+#pragma unroll
+                for (int b = a; b < D; ++b)
+                    M[a * D + b].fold();
+        }
+    }
+    const double scale = pr.factor * cutoff * fx::pow2(31 - 3 - fx::kListBits + volume_unit(f.Vol));
+#pragma unroll
+    for (int a = 0; a < D; ++a)
+#pragma unroll
+        for (int b = a; b < D; ++b)
+        {
+            fx::group_sum<LANES>(M[a * D + b]);
+            if (g.leads())
+                f.B[(a * D + b) * n + i] = M[a * D + b].value() * scale;
+        }
+}
+
+// The same sum over the wall neighbours, kWallLanes threads per particle that has any.
+template <int D>
+__global__ void __launch_bounds__(kBlock) k_ck_wall_matrix(size_t n, size_t n_active,
+                                                           const uint32_t *__restrict__ active, CKFluid f, CKWall w,
+                                                           Lists wl, TabK t, double *__restrict__ sum)
+{
+    __shared__ double rows[kIntervals * kRow];
+    load_rows(rows, t.dw);
+    Group<kWallLanes> g;
+    if (g.i >= n_active)
+        return;
+    g.i = active[g.i];
+    double x_i[3], r[3], inv, M[D * D];
+    for (int k = 0; k < D * D; ++k)
+        M[k] = 0.0;
+    load_point<D>(f.pos, n, g.i, x_i);
+    for_each_neighbor(wl, g, [&](uint32_t j) {
+        const double n2 = separation<D>(x_i, w.pos, w.nw, j, r, inv);
+        const double k = (tabulated(rows, (n2 * inv) * t.inv_step) * w.Vol[j]) * inv;
+#pragma unroll
+        for (int a = 0; a < D; ++a)
+        {
+            const double ka = k * r[a];
+#pragma unroll
+            for (int b = a; b < D; ++b)
+                M[a * D + b] = fma(ka, r[b], M[a * D + b]);
+        }
+    });
+    int c = 0;
+#pragma unroll
+    for (int a = 0; a < D; ++a)
+#pragma unroll
+        for (int b = a; b < D; ++b, ++c)
+        {
+            const double v = g.sum(M[a * D + b]);
+            if (g.leads())
+                sum[c * n + g.i] = v;
+        }
+}
+
+// The matrix from its sums, one thread per particle (about 200 FP64 instructions).
+template <int D>
+__global__ void __launch_bounds__(kBlock)
+    k_ck_correction_finish(size_t n, CKFluid f, const uint32_t *__restrict__ wall_count,
+                           const double *__restrict__ wall_sum, double alpha)
+{
+    const size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
+    if (i >= n)
+        return;
+    const bool wall = wall_count && wall_count[i] > 0;
+    double B[D * D];
+    int c = 0;
+#pragma unroll
+    for (int a = 0; a < D; ++a)
+#pragma unroll
+        for (int b = a; b < D; ++b, ++c)
+            B[a * D + b] = B[b * D + a] = -(f.B[(a * D + b) * n + i] + (wall ? wall_sum[c * n + i] : 0.0));
+    double determinant = det<D>(B);
+    double det_sqr = fmax(alpha - determinant, 0.0);
+    // inverseTikhonov (vector_functions.h:199-203): (B^T B + eps I)^-1 B^T, eps = SqrtEps
+    double BtB[D * D], Inv[D * D];
+    for (int a = 0; a < D; ++a)
+        for (int b = 0; b < D; ++b)
+        {
+            double sum = 0;
+            for (int k = 0; k < D; ++k)
+                sum += B[k * D + a] * B[k * D + b];
+            BtB[a * D + b] = sum + (a == b ? 1.0e-8 : 0.0);
+        }
+    inverse<D>(BtB, Inv);
+    double weight = determinant / (determinant + det_sqr);
+    double X[D * D], T[D * D];
+    for (int a = 0; a < D; ++a)
+        for (int b = 0; b < D; ++b)
+        {
+            double sum = 0;
+            for (int k = 0; k < D; ++k)
+                sum += Inv[a * D + k] * B[b * D + k];
+            X[a * D + b] = sum;
+        }
+    // One step of refinement, X += Inv (B^T (I - B X) - eps X); with the diagonal product first
+    // I - B X loses nothing.  Error of the matrix against extended precision (90,000 particles)
+    // 3.3e-16 -> 2.65e-16; FP64 sums with a division per pair, without it: 3.5e-16.
+    for (int a = 0; a < D; ++a)
+        for (int b = 0; b < D; ++b)
+        {
+            double v = fma(-B[a * D + a], X[a * D + b], a == b ? 1.0 : 0.0);
+            for (int k = 0; k < D; ++k)
+                if (k != a)
+                    v = fma(-B[a * D + k], X[k * D + b], v);
+            T[a * D + b] = v;
+        }
+    for (int b = 0; b < D; ++b)
+    {
+        double r[D];
+        for (int a = 0; a < D; ++a)
+        {
+            r[a] = -1.0e-8 * X[a * D + b];
+            for (int k = 0; k < D; ++k)
+                r[a] = fma(B[k * D + a], T[k * D + b], r[a]);
+        }
+        for (int a = 0; a < D; ++a)
+        {
+            double v = 0.0;
+            for (int k = 0; k < D; ++k)
+                v = fma(Inv[a * D + k], r[k], v);
+            f.B[(a * D + b) * n + i] = weight * (X[a * D + b] + v) + (1.0 - weight) * (a == b ? 1.0 : 0.0);
+        }
+    }
+}
+
 // FreeSurfaceIndicationCK<Inner<WithUpdate>, Contact<>> (surface_indication_ck.hpp:49-150):
 // position divergence -sum dW V r over the inner neighbours with the spatial-temporal rule
 // (a particle below the threshold that was not a surface particle and has no previous
@@ -1093,23 +1283,50 @@ __global__ void __launch_bounds__(kBlock, 4)
 // than h lies below it; the previous indicator takes the new value.
 template <int D, int LANES>
 __global__ void __launch_bounds__(kBlock)
-    k_ck_indication_inner(size_t n, CKFluid f, Lists in, TabK t, const int *__restrict__ prev,
-                          double *__restrict__ pos_div, double thr)
+    k_ck_indication_inner(size_t n, CKFluid f, Lists in, CKPairs pr, fx::Fixed fp, TabK t, double cutoff,
+                          const int *__restrict__ prev, double *__restrict__ pos_div, double thr)
 {
     __shared__ double rows[kIntervals * kRow];
-    load_rows(rows, t.dw);
+    const bool general = pr.general || __ldcg(fp.flag) == fp.epoch;
+    if (general)
+        load_rows(rows, t.dw);
     const Group<LANES> g;
     const size_t i = g.i;
     if (i >= n)
         return;
-    double pd = 0.0, x_i[3], r[3], inv;
-    load_point<D>(f.pos, n, i, x_i);
-    for_each_neighbor(in, g, [&](uint32_t j) {
-        const double n2 = separation<D>(x_i, f.pos, n, j, r, inv);
-        const double len = n2 * inv;
-        pd -= tabulated(rows, len * t.inv_step) * f.Vol[j] * len;
-    });
-    pd = g.sum(pd);
+    double pd = 0.0;
+    if (general)
+    {
+        double x_i[3], r[3], inv;
+        load_point<D>(f.pos, n, i, x_i);
+        for_each_neighbor(in, g, [&](uint32_t j) {
+            const double n2 = separation<D>(x_i, f.pos, n, j, r, inv);
+            const double len = n2 * inv;
+            pd -= tabulated(rows, len * t.inv_step) * f.Vol[j] * len;
+        });
+        pd = g.sum(pd);
+    }
+    else
+    {
+        fx::Sum S;
+        int folded = 0;
+        const unsigned cnt = min(pr.count[i], pr.cap);
+        for (unsigned s = g.sub; s < cnt; s += LANES)
+        {
+            const size_t slot = size_t(s) * n + i;
+            const uint32_t j = pr.J[slot];
+            if (!entry_ok(in, j))
+                continue;
+            S.m += moment(pr.at.load<D>(slot).k, __ldg(fp.value + j), pr.r[slot]);
+            if (++folded == fx::kFold)
+            {
+                folded = 0;
+                S.fold();
+            }
+        }
+        fx::group_sum<LANES>(S);
+        pd = -S.value() * (pr.factor * cutoff * fx::pow2(volume_unit(f.Vol) - 3));
+    }
     if (!g.leads())
         return;
     if (pd < thr && prev[i] != 1)
@@ -1124,18 +1341,19 @@ __global__ void __launch_bounds__(kBlock)
     pos_div[i] = pd;
 }
 
-template <int D, int LANES>
+template <int D>
 __global__ void __launch_bounds__(kBlock)
-    k_ck_indication_contact(size_t n, CKFluid f, CKWall w, Lists wl, TabK t, double *__restrict__ pos_div)
+    k_ck_indication_contact(size_t n, size_t n_active, const uint32_t *__restrict__ active, CKFluid f, CKWall w,
+                            Lists wl, TabK t, double *__restrict__ pos_div)
 {
     __shared__ double rows[kIntervals * kRow];
     load_rows(rows, t.dw);
-    const Group<LANES> g;
-    const size_t i = g.i;
-    if (i >= n)
+    Group<kWallLanes> g;
+    if (g.i >= n_active)
         return;
+    g.i = active[g.i];
     double pd = 0.0, x_i[3], r[3], inv;
-    load_point<D>(f.pos, n, i, x_i);
+    load_point<D>(f.pos, n, g.i, x_i);
     for_each_neighbor(wl, g, [&](uint32_t j) {
         const double n2 = separation<D>(x_i, w.pos, w.nw, j, r, inv);
         const double len = n2 * inv;
@@ -1143,10 +1361,9 @@ __global__ void __launch_bounds__(kBlock)
     });
     pd = g.sum(pd);
     if (g.leads())
-        pos_div[i] += pd;
+        pos_div[g.i] += pd;
 }
 
-// The distance is formed only for the neighbours below the threshold.
 template <int D>
 __global__ void k_ck_indication_update(size_t n, CKFluid f, Lists in, const double *__restrict__ pos_div,
                                        int *__restrict__ indicator, int *__restrict__ prev, double thr, double h)
@@ -1410,10 +1627,26 @@ int sweep_lanes(sphx_ctx ctx, int dim, size_t n)
         SPHX_LAUNCHED((b)->ctx);                                                                                       \
     } while (0)
 
-// The pair geometry of the relation's current lists, made on the first half step after an
-// update, and the record buffer of a half step with a fresh epoch for its verdict.
-static int ck_pairs(sphx_relation rel, const CKFluid &f, const TabK &t, const CKParams &k, int half, CKPairs &pr,
-                    fx::Fixed &fixed)
+// Launch over the particles with wall neighbours, kWallLanes threads each.
+#define CK_WALL(wall, KERNEL, ...)                                                                                     \
+    do                                                                                                                 \
+    {                                                                                                                  \
+        if ((wall) && (wall)->n_active > 0)                                                                            \
+        {                                                                                                              \
+            const unsigned grid_ = grid_for((wall)->n_active * kWallLanes, kBlock);                                    \
+            if ((wall)->src->dim == 2)                                                                                 \
+                KERNEL<2><<<grid_, kBlock, 0, (wall)->ctx->stream>>>((wall)->src->n, (wall)->n_active, (wall)->active, \
+                                                                     __VA_ARGS__);                                     \
+            else                                                                                                       \
+                KERNEL<3><<<grid_, kBlock, 0, (wall)->ctx->stream>>>((wall)->src->n, (wall)->n_active, (wall)->active, \
+                                                                     __VA_ARGS__);                                     \
+            SPHX_LAUNCHED((wall)->ctx);                                                                                \
+        }                                                                                                              \
+    } while (0)
+
+// The pair geometry of the relation's current lists, made on first use after an update
+// (summed: with the inner part of the compression sum in the same pass).
+static int ck_geometry(sphx_relation rel, const CKFluid &f, const TabK &t, CKPairs &pr, bool summed)
 {
     sphx_ctx ctx = rel->ctx;
     const int D = rel->src->dim;
@@ -1422,22 +1655,49 @@ static int ck_pairs(sphx_relation rel, const CKFluid &f, const TabK &t, const CK
     {
         SPHX_CUDA(cudaMalloc(&rel->ck_pos, n * D * sizeof(double)));
         SPHX_CUDA(cudaMalloc(&rel->ck_value, n * Rec1<3>::words * sizeof(long long)));
+        SPHX_CUDA(cudaMalloc(&rel->ck_r, slots * sizeof(int2)));
         if (D == 2)
             SPHX_CUDA(cudaMalloc(&rel->ck_k, slots * sizeof(int2)));
         SPHX_CUDA(cudaMalloc(&rel->ck_rec, slots * (D == 2 ? 1 : 2) * sizeof(int4)));
         rel->ck_version = 0;
     }
     pr = CKPairs{rel->count, rel->j, fx::EntryStore{rel->ck_rec, rel->ck_k}, unsigned(rel->cap),
-                 uint32_t(rel->tgt->n), wendland(D, rel->h).factor_dW, rel->ck_pos,
-                 rel->cap > int(fx::kMaxCap) || !(k.slope * k.inv_c0_ave >= 0.0)};
-    if (rel->ck_version != rel->version)
-    {
-        const double inv_factor = 1.0 / pr.factor;
-        CK_SWEEP(k_ck_pairs, D, ctx, n, n, f.pos, lists_of(rel), t, inv_factor, pr.at, rel->ck_pos);
-        rel->ck_version = rel->version;
-    }
+                 uint32_t(rel->tgt->n), wendland(D, rel->h).factor_dW, rel->ck_pos, rel->ck_r,
+                 rel->cap > int(fx::kMaxCap)};
+    if (rel->ck_version == rel->version)
+        return SPHX_OK;
+    const double inv_factor = 1.0 / pr.factor, inv_cutoff = 0.5 / rel->h;
+    if (summed)
+        CK_SWEEP(k_ck_pairs_sum, D, ctx, n, n, f, lists_of(rel), t, inv_factor, inv_cutoff, pr.at, rel->ck_r,
+                 rel->ck_pos);
+    else
+        CK_SWEEP(k_ck_pairs, D, ctx, n, n, f, lists_of(rel), t, inv_factor, inv_cutoff, pr.at, rel->ck_r, rel->ck_pos);
+    rel->ck_version = rel->version;
+    return SPHX_OK;
+}
+
+// The geometry and the record buffer of a sweep with a fresh epoch for its verdict.
+static int ck_pairs(sphx_relation rel, const CKFluid &f, const TabK &t, int half, CKPairs &pr, fx::Fixed &fixed)
+{
+    SPHX_TRY(ck_geometry(rel, f, t, pr, false));
     fixed = fx::Fixed{rel->ck_value, rel->fx_flag + half, ++rel->fx_epoch[half],
                       reinterpret_cast<unsigned long long *>(rel->fx_flag + 4)};
+    return SPHX_OK;
+}
+
+// CompressionSummation: with the pair geometry where that is due anyway, else by itself.
+static int ck_summed(sphx_relation inner, sphx_relation wall, const CKFluid &f, const CKWall &w, const TabK &t)
+{
+    sphx_body b = inner->src;
+    const size_t n = b->n;
+    if (inner->ck_version != inner->version)
+    {
+        CKPairs pr{};
+        SPHX_TRY(ck_geometry(inner, f, t, pr, true));
+        CK_WALL(wall, k_ck_wall_summation, f, w, lists_of(wall), t);
+        return SPHX_OK;
+    }
+    CK_SWEEP(k_ck_compression_summation, b->dim, b->ctx, n, n, f, w, lists_of(inner), lists_of(wall), t);
     return SPHX_OK;
 }
 
@@ -1473,8 +1733,9 @@ extern "C" int sphx_ck_density_regularization(sphx_relation inner, sphx_relation
     size_t n = b->n;
     if (n == 0)
         return SPHX_OK;
-    CK_SWEEP(k_ck_regularization, b->dim, b->ctx, n, n, f, w, lists_of(inner), lists_of(wall),
-                make_tab(b->dim, inner->h), p->rho0);
+    SPHX_TRY(ck_summed(inner, wall, f, w, make_tab(b->dim, inner->h)));
+    // the post-state DensityRegularization<FreeSurface>
+    CK_DISPATCH(b, k_ck_free_surface_regularization, grid_for(n, kBlock), n, f, p->rho0);
     return SPHX_OK;
 }
 
@@ -1489,8 +1750,7 @@ extern "C" int sphx_ck_compression_summation(sphx_relation inner, sphx_relation 
     size_t n = b->n;
     if (n == 0)
         return SPHX_OK;
-    CK_SWEEP(k_ck_compression_summation, b->dim, b->ctx, n, n, f, w, lists_of(inner), lists_of(wall),
-                make_tab(b->dim, inner->h), 0.0);
+    SPHX_TRY(ck_summed(inner, wall, f, w, make_tab(b->dim, inner->h)));
     return SPHX_OK;
 }
 
@@ -1541,8 +1801,15 @@ extern "C" int sphx_ck_linear_correction_matrix(sphx_relation inner, sphx_relati
     size_t n = b->n;
     if (n == 0)
         return SPHX_OK;
-    CK_SWEEP(k_ck_correction, b->dim, b->ctx, n, n, f, w, lists_of(inner), lists_of(wall),
-                make_tab(b->dim, inner->h), alpha);
+    const TabK t = make_tab(b->dim, inner->h);
+    CKPairs pr{};
+    fx::Fixed fp{};
+    SPHX_TRY(ck_pairs(inner, f, t, 0, pr, fp));
+    CK_DISPATCH(b, k_ck_volumes, grid_for(n, kBlock), n, f, pr, fp);
+    CK_WALL(wall, k_ck_wall_matrix, f, w, lists_of(wall), t, wall->contact_sum);
+    CK_SWEEP(k_ck_correction_sums, b->dim, b->ctx, n, n, f, lists_of(inner), pr, fp, t, 2.0 * inner->h);
+    CK_DISPATCH(b, k_ck_correction_finish, grid_for(n, kBlock), n, f, wall ? wall->count : nullptr,
+                wall ? wall->contact_sum : nullptr, alpha);
     return SPHX_OK;
 }
 
@@ -1573,9 +1840,13 @@ extern "C" int sphx_ck_free_surface_indication(sphx_relation inner, sphx_relatio
     TabK t = make_tab(b->dim, inner->h);
     double *pos_div = f64(pd);
     int *indicator = static_cast<int *>(ind->dev), *previous = static_cast<int *>(prev->dev);
-    CK_SWEEP(k_ck_indication_inner, b->dim, b->ctx, n, n, f, lists_of(inner), t, previous, pos_div, thr);
-    if (wall)
-        CK_SWEEP(k_ck_indication_contact, b->dim, b->ctx, n, n, f, w, lists_of(wall), t, pos_div);
+    CKPairs pr{};
+    fx::Fixed fp{};
+    SPHX_TRY(ck_pairs(inner, f, t, 0, pr, fp));
+    CK_DISPATCH(b, k_ck_volumes, grid_for(n, kBlock), n, f, pr, fp);
+    CK_SWEEP(k_ck_indication_inner, b->dim, ctx, n, n, f, lists_of(inner), pr, fp, t, 2.0 * inner->h, previous, pos_div,
+             thr);
+    CK_WALL(wall, k_ck_indication_contact, f, w, lists_of(wall), t, pos_div);
     CK_DISPATCH(b, k_ck_indication_update, grid_for(n, kBlock), n, f, lists_of(inner), pos_div, indicator, previous,
                 thr, inner->h);
     return SPHX_OK;
@@ -1599,7 +1870,7 @@ extern "C" int sphx_ck_acoustic_step_1st_half(sphx_relation inner, sphx_relation
     const TabK t = make_tab(b->dim, inner->h);
     CKPairs pr{};
     fx::Fixed fp{};
-    SPHX_TRY(ck_pairs(inner, f, t, k, 0, pr, fp));
+    SPHX_TRY(ck_pairs(inner, f, t, 0, pr, fp));
     CK_DISPATCH(b, k_ck_init1, grid_for(n, kBlock), n, f, k, dt, pr, fp);
     SPHX_TRY((ck_wall_terms<1>(wall, f, w, t, k)));
     CK_SWEEP(k_ck_interact1, b->dim, b->ctx, n, n, f, lists_of(inner), pr, fp, t, k, dt,
@@ -1626,7 +1897,8 @@ extern "C" int sphx_ck_acoustic_step_2nd_half(sphx_relation inner, sphx_relation
     sphx_ctx ctx = b->ctx;
     CKPairs pr{};
     fx::Fixed fv{};
-    SPHX_TRY(ck_pairs(inner, f, t, k, 1, pr, fv));
+    SPHX_TRY(ck_pairs(inner, f, t, 1, pr, fv));
+    pr.general = pr.general || !(k.slope * k.inv_c0_ave >= 0.0);
     if (b->dim == 2)
         fx::k_largest_velocity<2><<<red_grid(ctx, n), kBlock, 0, ctx->stream>>>(n, f.vel, fv);
     else

@@ -427,6 +427,8 @@ void sphx_relation_s::release()
     cudaFree(wsum);
     cudaFree(ck_rec);
     cudaFree(ck_k);
+    cudaFree(ck_r);
+    ck_r = nullptr;
     cudaFree(ck_pos);
     cudaFree(ck_value);
     ck_rec = nullptr;
@@ -478,7 +480,7 @@ int sphx_relation_s::allocate(int new_cap, size_t n)
         SPHX_CUDA(cudaMalloc(&dW, slots * sizeof(double)));
         SPHX_CUDA(cudaMalloc(&e, slots * dim * sizeof(double)));
         SPHX_CUDA(cudaMalloc(&active, nn * sizeof(uint32_t)));
-        SPHX_CUDA(cudaMalloc(&contact_sum, nn * (dim + 1) * sizeof(double)));
+        SPHX_CUDA(cudaMalloc(&contact_sum, nn * (dim == 2 ? 3 : 6) * sizeof(double)));
     }
     if (store_r)
         SPHX_CUDA(cudaMalloc(&r, slots * sizeof(double)));

@@ -171,11 +171,12 @@ struct sphx_relation_s
     uint32_t fx_epoch[3] = {0, 0, 0};
     longlong4_32a *fx_pos = nullptr; // cell-list entries: position in fixed point, particle
     size_t fx_pos_cap = 0;
-    // CK methods (ck.cu): the tabulated kernel derivative and unit vector of the pairs of list
-    // `ck_version`, made from the positions ck_pos, and the particle records of a sweep
+    // CK methods (ck.cu): the tabulated kernel derivative, unit vector and distance (over 2 h) of
+    // the pairs of list `ck_version`, made from the positions ck_pos, and the particle records of
+    // a sweep
     uint64_t version = 0, ck_version = 0;
     int4 *ck_rec = nullptr;
-    int2 *ck_k = nullptr;
+    int2 *ck_k = nullptr, *ck_r = nullptr;
     double *ck_pos = nullptr;
     long long *ck_value = nullptr;
     int reserve_positions(size_t n);
@@ -183,7 +184,7 @@ struct sphx_relation_s
     // order) and a workspace for their sums.
     uint32_t *active = nullptr;
     size_t n_active = 0;
-    double *contact_sum = nullptr; // (dim + 1) x n_src
+    double *contact_sum = nullptr; // 3 x n_src (2D), 6 x n_src (3D)
     int allocate(int cap, size_t n_src);
     void release();
 };

@@ -65,3 +65,43 @@ def test_fixed_point_matches_general_path(case, speed, rate):
     a, b = (half_steps(case, speed, rate, nudge) for nudge in (False, True))
     for k in OUT:
         assert np.max(np.abs(a[k] - b[k])) <= TOL * max(np.max(np.abs(b[k])), 1e-300), k
+
+
+def once_per_step(case, nudge, uneven):
+    """Compression sum with the pair geometry, then correction and indication from it."""
+    sim = DamBreakCKNested(case)
+    b, rng = sim.water_block, np.random.default_rng(6)
+    n, d = b.n, case.dim
+    x = b.download("Position").reshape(n, d) + rng.uniform(-0.2, 0.2, (n, d)) * case.dp
+    b.upload("Position", x)
+    b.updateCellLinkedList()
+    sim.fp64.water_block_inner.updateConfiguration()
+    sim.fp64.water_wall_contact.updateConfiguration()
+    sim.regularization.exec()
+    out = {"fused sum": b.download("CompressionSummation")}
+    if nudge:
+        x[n // 2, 0] = np.nextafter(x[n // 2, 0], np.inf)
+        b.upload("Position", x)
+    sim.setup.exec()
+    if uneven:  # volumes of a factor of two around the first particle's
+        b.upload("VolumetricMeasure", b.download("VolumetricMeasure") * rng.uniform(0.7, 1.4, n))
+    sim.regularization.exec()
+    sim.correction.exec()
+    for k in ("first", "again"):
+        sim.indication.exec()
+        out[k] = b.download("PositionDivergence")
+        out[k + " indicator"] = b.download("Indicator")
+    out["sum"] = b.download("CompressionSummation")
+    out["correction"] = b.download("LinearCorrectionMatrix")
+    return out
+
+
+@pytest.mark.parametrize("case", CASES, ids=lambda c: c.name)
+@pytest.mark.parametrize("uneven", [False, True])
+def test_once_per_step_matches_general_path(case, uneven):
+    """The same tolerance: 3e-14 for a sum, and a correction matrix (the regularised inverse of
+    one) of a condition number squared below 1000."""
+    a, b = (once_per_step(case, nudge, uneven) for nudge in (False, True))
+    for k in a:
+        assert np.max(np.abs(a[k] - b[k])) <= TOL * np.max(np.abs(b[k])), k
+    assert np.max(np.abs(a["fused sum"] - a["sum"])) <= TOL * np.max(np.abs(a["sum"]))
