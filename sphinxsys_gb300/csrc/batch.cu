@@ -435,7 +435,9 @@ __global__ void k_b_initial_max(size_t n, const uint32_t *__restrict__ starts, i
         return;
     int b = find_instance(starts, count, uint32_t(i));
     double vm, am;
-    initial_max<D>(i, n, inst[b].p, inst[b].gd, f, &vm, &am);
+    double v2, a2;
+    initial_squares<D>(i, n, inst[b].p, inst[b].gd, f, v2, a2);
+    initial_max(inst[b].p, v2, a2, &vm, &am);
     atomicMax(&run[b].ac, ordered_bits(vm));
     atomicMax(&run[b].adv, ordered_bits(am));
 }

@@ -1653,10 +1653,14 @@ static int ck_geometry(sphx_relation rel, const CKFluid &f, const TabK &t, CKPai
     const size_t n = rel->n_src, slots = size_t(rel->cap) * n;
     if (!rel->ck_rec)
     {
-        SPHX_CUDA(cudaMalloc(&rel->ck_pos, n * D * sizeof(double)));
-        SPHX_CUDA(cudaMalloc(&rel->ck_value, n * Rec1<3>::words * sizeof(long long)));
-        SPHX_CUDA(cudaMalloc(&rel->ck_r, slots * sizeof(int2)));
-        if (D == 2)
+        // an earlier attempt may have run out of memory half way
+        if (!rel->ck_pos)
+            SPHX_CUDA(cudaMalloc(&rel->ck_pos, n * D * sizeof(double)));
+        if (!rel->ck_value)
+            SPHX_CUDA(cudaMalloc(&rel->ck_value, n * Rec1<3>::words * sizeof(long long)));
+        if (!rel->ck_r)
+            SPHX_CUDA(cudaMalloc(&rel->ck_r, slots * sizeof(int2)));
+        if (D == 2 && !rel->ck_k)
             SPHX_CUDA(cudaMalloc(&rel->ck_k, slots * sizeof(int2)));
         SPHX_CUDA(cudaMalloc(&rel->ck_rec, slots * (D == 2 ? 1 : 2) * sizeof(int4)));
         rel->ck_version = 0;

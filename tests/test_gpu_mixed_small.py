@@ -7,6 +7,7 @@ import numpy as np
 import pytest
 
 from sphinxsys_gb300 import cases
+from sphinxsys_gb300 import native as N
 from sphinxsys_gb300.dambreak import MixedPrecisionDamBreak
 from sphinxsys_gb300.taylor_green import MixedPrecisionTaylorGreen
 
@@ -50,3 +51,22 @@ def test_plan_matches_step_by_step(case):
 @pytest.mark.parametrize("case", [cases.taylor_green_2d(50), cases.taylor_green_3d(24)], ids=lambda c: c.name)
 def test_periodic_plan_matches_step_by_step(case):
     same(advance(MixedPrecisionTaylorGreen(case), 6, False), advance(MixedPrecisionTaylorGreen(case), 6, True))
+
+
+@pytest.mark.parametrize("case", [cases.dambreak_2d(0.1), cases.dambreak_3d(0.12)], ids=lambda c: c.name)
+def test_download_widens_every_float_exactly(case):
+    """The download converts by integer instructions: zeros, subnormals and the limits too."""
+    sim = MixedPrecisionDamBreak(case)
+    body = sim.fp64.water_block
+    special = np.array([0.0, -0.0, 1e-45, -1e-45, 1.1754942e-38, 1.17549435e-38, -5e-39, 3.4028235e38, -1.0, 0.1, 7e-30],
+                       np.float32)
+    values = np.resize(special, (body.n, case.dim)).astype(np.float64)
+    for k in ("Velocity", "Force"):
+        body.upload(k, values)
+    N.call("sphx_mp_upload", sim.handle, body.handle)
+    for k in ("Velocity", "Force"):
+        body.upload(k, np.ones_like(values))
+    sim.sync_fp64()
+    for k in ("Velocity", "Force"):
+        got = np.asarray(body.download(k)).reshape(values.shape)
+        assert np.array_equal(got, values) and np.array_equal(np.signbit(got), np.signbit(values)), k
