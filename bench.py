@@ -129,11 +129,12 @@ def traffic_of(key):
 
 
 def bytes_fp64_second(n_fluid: int, n_wall_active: int, nnz: int) -> int:
-    """Integration2ndHalf, FP64 3D: 136 B per fluid particle (read x, v, rho, drho, Vol;
-    write x, rho, drho, F), 80 B per active wall particle (x, V, v_ave, n), 36 B per stored
-    pair: the neighbour index and the configuration-time dW (8 B) and e (24 B) the classic
-    neighbourhood keeps for the whole advection step."""
-    return 136 * n_fluid + 80 * n_wall_active + 36 * nnz
+    """Integration2ndHalf, FP64 3D: 168 B per fluid particle (read x, v, rho, drho, Vol;
+    write x, rho, drho, F; the fixed-point velocity and volume record, 32 B), 80 B per
+    active wall particle (x, V, v_ave, n), 36 B per stored pair: the neighbour index and the
+    configuration-time dW (8 B) and e (24 B) the classic neighbourhood keeps for the whole
+    advection step."""
+    return 168 * n_fluid + 80 * n_wall_active + 36 * nnz
 
 
 def bytes_mp_second(n_fluid: int, n_wall_active: int, nnz: int) -> int:
@@ -341,7 +342,7 @@ def fp64_leg(args, torch, local):
     out = {"workload": case.name, "n_fluid": n, "dtype": "f64", "value": n * subs / el,
            "ms_per_step": 1e3 * el / args.fp64_steps, "steps": args.fp64_steps, "acoustic_substeps": subs,
            "gpu_launches": int(launches),
-           "roofline": {"bound": "fp64 pipe (reported against hbm)", "achieved": achieved, "peak": hbm,
+           "roofline": {"bound": "issue and hbm (fixed-point sums; reported against hbm)", "achieved": achieved, "peak": hbm,
                         "unit": "GB/s", "frac": achieved / hbm, "traffic": traffic_of("k_interact_2nd"),
                         "kernel": "k_interact_2nd<3>", "algorithmic_bytes": alg, "kernel_ms": k_ms,
                         "peak_source": src}}
